@@ -28,6 +28,7 @@ SOURCES = [
     ("afile.cpp", []),
     ("api.cu", []),
     ("collide.cu", []),
+    ("collide_mma.cu", []),
     ("collide_tc.cu", []),
     ("adjoint.cu", []),
     ("noalloc.cu", []),

@@ -205,7 +205,7 @@ int vjp_device(Ctx *c, const double *d_f, const double *d_v, double *d_g, int pr
     a.fg = nullptr;
     if (gf) {
         const void *fg = nullptr;
-        if ((rc = f_local_major(c, d_f, 1, false, &fg))) return rc;
+        if ((rc = f_local_major(c, d_f, nullptr, 1, false, &fg))) return rc;
         a.fg = static_cast<const double *>(fg);
     }
     fn<<<dim3(1, slices * npsl, nchunks), 32 + dcta, smem, c->stream>>>(a);

@@ -297,8 +297,8 @@ static KernelFn pick_kernel_gf(int P, int mode)
         return k_collide_pipe<PV, MODE_BILINEAR, false, GF>;
     switch (P) {
         DGV_PICK(1)
-        DGV_PICK(8)
-        DGV_PICK(27)
+    case 8: return mode == MODE_F32C ? k_collide_pipe<8, MODE_F32C, false, GF> : nullptr;  // FP64: collide_mma.cu
+    case 27: return mode == MODE_F32C ? k_collide_pipe<27, MODE_F32C, false, GF> : nullptr;
     case 125:  // slices of 25 basis functions per CTA
         if (mode == MODE_F64) return k_collide_pipe<P_SLICE, MODE_F64, true, GF>;
         if (mode == MODE_F32C) return k_collide_pipe<P_SLICE, MODE_F32C, true, GF>;
@@ -371,20 +371,23 @@ int ensure_rows32(Ctx *c)
     return DGV_OK;
 }
 
-int f_local_major(Ctx *c, const double *d_f, int nvdf, bool f32, const void **out)
+int f_local_major(Ctx *c, const double *d_f, const double *d_g, int nvdf, bool f32, const void **out)
 {
     const Grid &g = c->grid;
-    int rc = ensure_buffer(c, &c->d_fg, &c->fg_bytes, (size_t)nvdf * g.N * (f32 ? sizeof(float) : sizeof(double)));
+    const size_t n = (size_t)nvdf * g.N, word = f32 ? sizeof(float) : sizeof(double);
+    int rc = ensure_buffer(c, &c->d_fg, &c->fg_bytes, (d_g ? 2 : 1) * n * word);
     if (rc) return rc;
-    const long long tot = (long long)nvdf * g.N;
-    const unsigned nblk = (unsigned)std::min<long long>((tot + 255) / 256, 148LL * 16);
-    if (f32)
-        k_f_local_major<float><<<nblk, 256, 0, c->stream>>>(d_f, reinterpret_cast<float *>(c->d_fg), g.N, g.Nc, g.P,
-                                                            nvdf);
-    else
-        k_f_local_major<double><<<nblk, 256, 0, c->stream>>>(d_f, c->d_fg, g.N, g.Nc, g.P, nvdf);
-    DGV_CUDA(c, cudaGetLastError());
-    count_launches(c, 1);
+    const unsigned nblk = (unsigned)std::min<long long>(((long long)n + 255) / 256, 148LL * 16);
+    for (int k = 0; k < (d_g ? 2 : 1); k++) {
+        const double *src = k ? d_g : d_f;
+        if (f32)
+            k_f_local_major<float><<<nblk, 256, 0, c->stream>>>(src, reinterpret_cast<float *>(c->d_fg) + k * n, g.N, g.Nc,
+                                                                g.P, nvdf);
+        else
+            k_f_local_major<double><<<nblk, 256, 0, c->stream>>>(src, c->d_fg + k * n, g.N, g.Nc, g.P, nvdf);
+        DGV_CUDA(c, cudaGetLastError());
+        count_launches(c, 1);
+    }
     *out = c->d_fg;
     return DGV_OK;
 }
@@ -465,7 +468,7 @@ static int run_collide(Ctx *c, const double *d_f, const double *d_f2, double *d_
     a.Pt = g.P; a.npsl = p_slices(g.P);
     a.wait_ns = wait_limit_ns(c);
     a.fg = nullptr;
-    if (sh.gf && (rc = f_local_major(c, d_f, nvdf, mode == MODE_F32C, &a.fg))) return rc;
+    if (sh.gf && (rc = f_local_major(c, d_f, nullptr, nvdf, mode == MODE_F32C, &a.fg))) return rc;
     // VDF fastest: the CTAs resident at one time work on the same chunk of
     // rows for different VDFs, so each row is fetched from HBM once and then
     // served from L2
@@ -540,8 +543,13 @@ int collide_device(Ctx *c, const double *d_f, double *d_q, int nvdf, int precisi
     if (precision == DGV_PREC_TC) return collide_tc_device(c, d_f, d_q, nvdf, scale);
     if (precision != DGV_PREC_F64 && precision != DGV_PREC_F32C)
         return set_err(c, DGV_EINVAL, "collide: unknown precision");
-    int nch = choose_chunks(c, d_f, nullptr, d_q, nvdf, precision, 0, c->grid.Nc);
-    int rc = run_collide(c, d_f, nullptr, d_q, nvdf, precision, scale, nch, 0, c->grid.Nc);
+    int rc;
+    if (precision == DGV_PREC_F64 && mma_serves(c)) {
+        rc = collide_mma_device(c, d_f, nullptr, d_q, nvdf, scale, 0, c->grid.Nc);
+    } else {
+        const int nch = choose_chunks(c, d_f, nullptr, d_q, nvdf, precision, 0, c->grid.Nc);
+        rc = run_collide(c, d_f, nullptr, d_q, nvdf, precision, scale, nch, 0, c->grid.Nc);
+    }
     if (rc) return rc;
     if (c->project) return project_device(c, d_q, nvdf);
     return DGV_OK;
@@ -554,6 +562,8 @@ int collide_cells_device(Ctx *c, const double *d_f, double *d_q, int nvdf, int p
         return set_err(c, DGV_EUNSUP, "collide_cells: FP64 or FP32-compensated only");
     if (cell0 < 0 || cell1 > c->grid.Nc || cell0 >= cell1)
         return set_err(c, DGV_ERANGE, "collide_cells: cell range outside [0, Nc) or empty");
+    if (precision == DGV_PREC_F64 && mma_serves(c))
+        return collide_mma_device(c, d_f, nullptr, d_q, nvdf, 1.0, cell0, cell1);
     int nch = choose_chunks(c, d_f, nullptr, d_q, nvdf, precision, cell0, cell1);
     return run_collide(c, d_f, nullptr, d_q, nvdf, precision, 1.0, nch, cell0, cell1);
 }
@@ -562,6 +572,7 @@ int jvp_device(Ctx *c, const double *d_f, const double *d_df, double *d_q, int p
 {
     if (!c->lay.blk) return set_err(c, DGV_ESTATE, "jvp: no A-arrays loaded");
     if (precision != DGV_PREC_F64) return set_err(c, DGV_EUNSUP, "jvp: the mixed-terms kernel computes in FP64 only");
+    if (mma_serves(c)) return collide_mma_device(c, d_f, d_df, d_q, 1, 1.0, 0, c->grid.Nc);
     int nch = choose_chunks(c, d_f, d_df, d_q, 1, DGV_PREC_F64, 0, c->grid.Nc);
     // the bilinear kernel sums 2/w * A * (f g + g f) / 2 * 2: the reduce
     // kernel's factor 2 is the reference's "2*fc/w" (collision_mod.f90:326)

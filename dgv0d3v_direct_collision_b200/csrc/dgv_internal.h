@@ -45,6 +45,23 @@ struct Grid {
 };
 int build_grid(const dgv_grid_desc &d, Grid &g, std::string &err);
 
+// Blocks with the same box of output cells and their stages (collide_mma.cu)
+struct MmaBox {
+    int lo[3], hi[3];
+    long long stage0, stage1;
+};
+
+// The units of a range of output cells (collide_mma.cu): device array, and per
+// unit the running cost, first stage and cost per stage; per number of ranges
+// the device array of their bounds
+struct MmaPlan {
+    void *units = nullptr;
+    int nunits = 0;
+    std::vector<long long> cost;
+    std::vector<int> first, last, per_stage, per_unit;
+    std::map<int, void *> bounds;
+};
+
 // Device copy of the A-arrays in the pair layout.
 //   rows64[pair] = { int32 o1, int32 o2, double v[P], pad }  (RD64 doubles)
 //   rows32[pair] = { int32 o1, int32 o2, float v[P], pad }   (RW32 words)
@@ -63,6 +80,11 @@ struct Layout {
     std::vector<double> h_work;       // per block: pairs x valid shifts
     // work partitions: nchunks -> device array of nchunks+1 block bounds
     std::map<int, int *> chunks;
+    // FP64 tensor instructions (built on first use): stages in box order, the
+    // boxes, and the units per range of output cells
+    void *mma_segs = nullptr, *mma_sfirst = nullptr;  // device
+    std::vector<MmaBox> mma_box;
+    std::map<std::pair<int, int>, MmaPlan> mma_plans;
     // tensor-core form (built on first use): per block ceil(count/64) chunk
     // records of split-fp16 value tiles, their first record per block, the
     // power-of-two value scale, and the block sets of one launch each
@@ -192,8 +214,9 @@ int release_layouts(Ctx *c, int mask);
 // the FP32 rows, rebuilt from the FP64 rows after a release
 int ensure_rows32(Ctx *c);
 // local-major copies f[v][l*Nc + cell] of nvdf VDFs (FP32 or FP64) in the
-// context's buffer, for the CUDA-core kernels that gather f from global memory
-int f_local_major(Ctx *c, const double *d_f, int nvdf, bool f32, const void **out);
+// context's buffer, for the kernels that gather f from global memory; with d_g
+// those of g follow
+int f_local_major(Ctx *c, const double *d_f, const double *d_g, int nvdf, bool f32, const void **out);
 // the limit of the kernels' bounded waits (DGV_OPT_WAIT_LIMIT_US, else 4 s)
 inline unsigned long long wait_limit_ns(const Ctx *c)
 {
@@ -221,6 +244,9 @@ int get_chunks(Ctx *c, int nchunks, int **d_bounds);
 // kernels (device pointers, ctx stream)
 int collide_device(Ctx *c, const double *d_f, double *d_q, int nvdf, int precision,
                    double scale);
+bool mma_serves(const Ctx *c);
+int collide_mma_device(Ctx *c, const double *d_f, const double *d_g, double *d_q, int nvdf, double scale, int cell0,
+                       int cell1);
 int collide_tc_device(Ctx *c, const double *d_f, double *d_q, int nvdf, double scale);
 int collide_cells_device(Ctx *c, const double *d_f, double *d_q, int nvdf, int precision, int cell0, int cell1);
 int jvp_device(Ctx *c, const double *d_f, const double *d_df, double *d_q, int precision);
