@@ -297,8 +297,6 @@ static KernelFn pick_kernel_gf(int P, int mode)
         return k_collide_pipe<PV, MODE_BILINEAR, false, GF>;
     switch (P) {
         DGV_PICK(1)
-    case 8: return mode == MODE_F32C ? k_collide_pipe<8, MODE_F32C, false, GF> : nullptr;  // FP64: collide_mma.cu
-    case 27: return mode == MODE_F32C ? k_collide_pipe<27, MODE_F32C, false, GF> : nullptr;
     case 125:  // slices of 25 basis functions per CTA
         if (mode == MODE_F64) return k_collide_pipe<P_SLICE, MODE_F64, true, GF>;
         if (mode == MODE_F32C) return k_collide_pipe<P_SLICE, MODE_F32C, true, GF>;
@@ -544,8 +542,8 @@ int collide_device(Ctx *c, const double *d_f, double *d_q, int nvdf, int precisi
     if (precision != DGV_PREC_F64 && precision != DGV_PREC_F32C)
         return set_err(c, DGV_EINVAL, "collide: unknown precision");
     int rc;
-    if (precision == DGV_PREC_F64 && mma_serves(c)) {
-        rc = collide_mma_device(c, d_f, nullptr, d_q, nvdf, scale, 0, c->grid.Nc);
+    if (mma_serves(c)) {
+        rc = collide_mma_device(c, d_f, nullptr, d_q, nvdf, precision, scale, 0, c->grid.Nc);
     } else {
         const int nch = choose_chunks(c, d_f, nullptr, d_q, nvdf, precision, 0, c->grid.Nc);
         rc = run_collide(c, d_f, nullptr, d_q, nvdf, precision, scale, nch, 0, c->grid.Nc);
@@ -562,8 +560,7 @@ int collide_cells_device(Ctx *c, const double *d_f, double *d_q, int nvdf, int p
         return set_err(c, DGV_EUNSUP, "collide_cells: FP64 or FP32-compensated only");
     if (cell0 < 0 || cell1 > c->grid.Nc || cell0 >= cell1)
         return set_err(c, DGV_ERANGE, "collide_cells: cell range outside [0, Nc) or empty");
-    if (precision == DGV_PREC_F64 && mma_serves(c))
-        return collide_mma_device(c, d_f, nullptr, d_q, nvdf, 1.0, cell0, cell1);
+    if (mma_serves(c)) return collide_mma_device(c, d_f, nullptr, d_q, nvdf, precision, 1.0, cell0, cell1);
     int nch = choose_chunks(c, d_f, nullptr, d_q, nvdf, precision, cell0, cell1);
     return run_collide(c, d_f, nullptr, d_q, nvdf, precision, 1.0, nch, cell0, cell1);
 }
@@ -572,7 +569,7 @@ int jvp_device(Ctx *c, const double *d_f, const double *d_df, double *d_q, int p
 {
     if (!c->lay.blk) return set_err(c, DGV_ESTATE, "jvp: no A-arrays loaded");
     if (precision != DGV_PREC_F64) return set_err(c, DGV_EUNSUP, "jvp: the mixed-terms kernel computes in FP64 only");
-    if (mma_serves(c)) return collide_mma_device(c, d_f, d_df, d_q, 1, 1.0, 0, c->grid.Nc);
+    if (mma_serves(c)) return collide_mma_device(c, d_f, d_df, d_q, 1, DGV_PREC_F64, 1.0, 0, c->grid.Nc);
     int nch = choose_chunks(c, d_f, d_df, d_q, 1, DGV_PREC_F64, 0, c->grid.Nc);
     // the bilinear kernel sums 2/w * A * (f g + g f) / 2 * 2: the reduce
     // kernel's factor 2 is the reference's "2*fc/w" (collision_mod.f90:326)

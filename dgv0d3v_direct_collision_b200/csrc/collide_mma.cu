@@ -57,10 +57,6 @@ constexpr int MM_THREADS = 32 * MM_WARPS;
 constexpr int MM_SP = 16;    // pairs per stage
 constexpr int MM_MT = 8;     // row tiles of 8 per unit
 constexpr int MM_MAXST = 4;  // ring stages per warp, at most
-// SM cycles of a stage per row tile, per stage, per unit and per tile at the
-// end of a unit: weights of the ranges' equal cost
-constexpr int MM_C_TILE = 66, MM_C_STAGE = 80, MM_C_UNIT = 3000, MM_C_FLUSH = 600;
-
 // One box of output cells and up to 8 * MM_MT of its cells: rows row0 ..
 // row0 + nrow - 1 of the box's cells in node order (u outer, w inner); the
 // stages [stage0, stage1) hold the pairs of all blocks with this box.
@@ -103,8 +99,9 @@ __device__ __forceinline__ int mma_cell(const MmaUnit &u, int r, int Mv, int Mw)
     return ((u.lo[0] + x) * Mv + u.lo[1] + v) * Mw + u.lo[2] + w;
 }
 
-// Walks the stages of one warp: every MM_WARPS-th stage of every unit of the
+// Walks the stages of one warp: every W-th stage of every unit of the
 // CTA's range.
+template <int W>
 struct MmaWalk {
     int u, s, end;
     __device__ __forceinline__ void enter(const MmaArgs &a, int2 b0, int2 b1, int warp)
@@ -118,7 +115,7 @@ struct MmaWalk {
     }
     __device__ __forceinline__ void next(const MmaArgs &a, int2 b0, int2 b1, int warp)
     {
-        s += MM_WARPS;
+        s += W;
         if (s < end) return;
         u++;
         enter(a, b0, b1, warp);
@@ -149,6 +146,103 @@ struct MmaF {
     {
         if constexpr (GF) return __ldg(g + q);
         else return lds_f64(g_s + q);
+    }
+};
+
+// One warp's stages: walks its range, keeps the ring of bulk copies full (one
+// copy per segment of a stage, lane k the k-th), and hands the stages out.  A
+// stage's segments are loaded one stage before their use, their range two
+// before: no load is waited for where it is issued.
+template <int W>
+struct MmaFetch {
+    unsigned char *ring;
+    uint64_t *full;
+    volatile int *cnt;
+    int2 b0, b1;
+    MmaWalk<W> pw;
+    unsigned long long ent = 0;    // this lane's segment of the next stage to issue
+    int nseg = 0, s0 = 0, s1 = 0;  // its segments; segment range of the stage after it
+    bool have = false, have2 = false, ok = true;
+    int warp, lane, islot = 0, cslot = 0, cphase = 0, inflight = 0;
+
+    __device__ __forceinline__ MmaFetch(const MmaArgs &a, unsigned char *smem, int w, int2 from, int2 to)
+        : b0(from), b1(to), warp(w), lane(threadIdx.x & 31)
+    {
+        ring = smem + warp * a.nst * MM_SP * a.rowb;
+        full = reinterpret_cast<uint64_t *>(smem + a.off_bar) + warp * MM_MAXST;
+        cnt = reinterpret_cast<volatile int *>(smem + a.off_bar + W * MM_MAXST * 8) + warp * MM_MAXST;
+        if (lane == 0) {
+            for (int s = 0; s < a.nst; s++) mbar_init(&full[s], 1);
+            fence_mbar_init();
+        }
+        __syncwarp();
+        pw.u = b0.x;
+        pw.enter(a, b0, b1, warp);
+        advance(a);
+        advance(a);
+        for (int s = 0; s < a.nst; s++) issue(a);
+    }
+    __device__ __forceinline__ void advance(const MmaArgs &a)
+    {
+        have = have2;
+        nseg = s1 - s0;
+        if (have && lane < nseg) ent = __ldg(a.segs + s0 + lane);
+        have2 = pw.u <= b1.x;
+        if (have2) {
+            s0 = __ldg(a.sfirst + pw.s);
+            s1 = __ldg(a.sfirst + pw.s + 1);
+            pw.next(a, b0, b1, warp);
+        }
+    }
+    __device__ __forceinline__ void issue(const MmaArgs &a)
+    {
+        if (!have) return;
+        const int off = (int)(ent >> 8 & 255ULL), len = (int)(ent & 255ULL);
+        const int n = __shfl_sync(0xffffffffu, off + len, nseg - 1);
+        if (lane == 0) {
+            cnt[islot] = n;
+            mbar_arrive_expect_tx(&full[islot], (uint32_t)(n * a.rowb));
+        }
+        if (lane < nseg)
+            bulk_g2s(ring + (islot * MM_SP + off) * a.rowb, a.rows + (size_t)(ent >> 16) * a.rowb,
+                     (uint32_t)(len * a.rowb), &full[islot]);
+        inflight++;
+        islot = islot + 1 == a.nst ? 0 : islot + 1;
+        advance(a);
+    }
+    // waits for the next stage: n = its pairs; false once a wait has given up
+    __device__ __forceinline__ bool wait(const MmaArgs &a, int &n)
+    {
+        if (ok) {
+            const bool got = mbar_wait(&full[cslot], cphase, a.err, a.wait_ns);
+            ok = __all_sync(0xffffffffu, got);
+        }
+        if (ok) n = cnt[cslot];
+        return ok;
+    }
+    __device__ __forceinline__ const unsigned char *stage(const MmaArgs &a) const { return ring + cslot * MM_SP * a.rowb; }
+    // done with it: its slot takes the next copy
+    __device__ __forceinline__ void done(const MmaArgs &a)
+    {
+        inflight--;
+        if (++cslot == a.nst) {
+            cslot = 0;
+            cphase ^= 1;
+        }
+        __syncwarp();  // every lane has read the slot
+        issue(a);
+    }
+    // after a wait that gave up: let the copies already issued land
+    __device__ __forceinline__ void drain(const MmaArgs &a)
+    {
+        if (ok) return;
+        for (; inflight > 0; inflight--) {
+            mbar_wait(&full[cslot], cphase, a.err, a.wait_ns);
+            if (++cslot == a.nst) {
+                cslot = 0;
+                cphase ^= 1;
+            }
+        }
     }
 };
 
@@ -202,62 +296,13 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_collide_mma(const __grid_cons
     extern __shared__ __align__(128) unsigned char smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int vdf = blockIdx.x, chunk = blockIdx.y;
-    const int stage_bytes = MM_SP * a.rowb;
-    unsigned char *ring = smem + warp * a.nst * stage_bytes;
     double *f_s = reinterpret_cast<double *>(smem + a.off_f), *g_s = reinterpret_cast<double *>(smem + a.off_g);
     double *red = reinterpret_cast<double *>(smem + a.off_red);  // [red_tiles][MM_WARPS][8][CW]
     __shared__ int rowcell[8 * MM_MT];
-    uint64_t *full = reinterpret_cast<uint64_t *>(smem + a.off_bar) + warp * MM_MAXST;
-    volatile int *cnt = reinterpret_cast<volatile int *>(smem + a.off_bar + MM_WARPS * MM_MAXST * 8) + warp * MM_MAXST;
     // the CTA's partial Q: in shared memory where that has room
     double *part = a.part_smem ? reinterpret_cast<double *>(smem + a.off_part)
                                : a.partial + ((size_t)vdf * a.nchunks + chunk) * ((size_t)a.ncell * P);
-    const int2 b0 = a.bounds[chunk], b1 = a.bounds[chunk + 1];
-
-    if (lane == 0) {
-        for (int s = 0; s < a.nst; s++) mbar_init(&full[s], 1);
-        fence_mbar_init();
-    }
-    __syncwarp();
-    // the warp's copies: one per segment of a stage, lane k the k-th.  A stage's
-    // segments are loaded one stage before their use, their range two before:
-    // no load is waited for where it is issued.
-    MmaWalk pw;
-    pw.u = b0.x;
-    pw.enter(a, b0, b1, warp);
-    unsigned long long ent = 0;  // this lane's segment of the next stage to issue
-    int nseg = 0, s0 = 0, s1 = 0;  // its segments; segment range of the stage after it
-    bool have = false, have2 = false;
-    auto advance = [&]() {
-        have = have2;
-        nseg = s1 - s0;
-        if (have && lane < nseg) ent = __ldg(a.segs + s0 + lane);
-        have2 = pw.u <= b1.x;
-        if (have2) {
-            s0 = __ldg(a.sfirst + pw.s);
-            s1 = __ldg(a.sfirst + pw.s + 1);
-            pw.next(a, b0, b1, warp);
-        }
-    };
-    advance();
-    advance();
-    int islot = 0, issued = 0;
-    auto issue = [&]() {
-        if (!have) return;
-        const int slot = islot, off = (int)(ent >> 8 & 255ULL), len = (int)(ent & 255ULL);
-        const int n = __shfl_sync(0xffffffffu, off + len, nseg - 1);
-        if (lane == 0) {
-            cnt[slot] = n;
-            mbar_arrive_expect_tx(&full[slot], (uint32_t)(n * a.rowb));
-        }
-        if (lane < nseg)
-            bulk_g2s(ring + slot * stage_bytes + off * a.rowb, a.rows + (size_t)(ent >> 16) * a.rowb,
-                     (uint32_t)(len * a.rowb), &full[slot]);
-        issued++;
-        islot = islot + 1 == a.nst ? 0 : islot + 1;
-        advance();
-    };
-    for (int s = 0; s < a.nst; s++) issue();
+    MmaFetch<MM_WARPS> fetch(a, smem, warp, a.bounds[chunk], a.bounds[chunk + 1]);
 
     if constexpr (!GF) {
         const double *f = a.f + (size_t)vdf * a.N;
@@ -281,11 +326,9 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_collide_mma(const __grid_cons
     F.f = GF ? a.fg + (size_t)vdf * a.N : nullptr;
     F.g = (GF && BIL) ? a.gg + (size_t)vdf * a.N : nullptr;
 
-    int it = 0, cslot = 0, cphase = 0;  // stages consumed; ring slot and phase of the next
-    bool ok = true;
-    for (int u = b0.x; u <= b1.x; u++) {
+    for (int u = fetch.b0.x; u <= fetch.b1.x; u++) {
         const MmaUnit un = a.units[u];
-        const int sa = u == b0.x ? b0.y : un.stage0, sb = u == b1.x ? b1.y : un.stage1;
+        const int sa = u == fetch.b0.x ? fetch.b0.y : un.stage0, sb = u == fetch.b1.x ? fetch.b1.y : un.stage1;
         if (sa >= sb) continue;  // the same in every warp
         const int nt = (un.nrow + 7) / 8;
         // the rows' cells: lane l has rows l and l + 32; rows past the last
@@ -306,27 +349,16 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_collide_mma(const __grid_cons
 #pragma unroll
             for (int t = 0; t < NTN; t++) acc[i][t][0] = acc[i][t][1] = 0.0;
         // the stages of this warp: sa + warp, sa + warp + MM_WARPS, ...
-        const int nmine = ok ? (sb - sa - warp + MM_WARPS - 1) / MM_WARPS : 0;
-#define DGV_MMA_CASE(NT)                                                                          \
-    case NT:                                                                                      \
-        for (int s = 0; s < nmine; s++) {                                                         \
-            const bool got = mbar_wait(&full[cslot], cphase, a.err, a.wait_ns);                   \
-            if (!__all_sync(0xffffffffu, got)) {                                                  \
-                ok = false;                                                                       \
-                break;                                                                            \
-            }                                                                                     \
-            const int n = cnt[cslot];                                                             \
-            const unsigned char *st = ring + cslot * stage_bytes;                                 \
-            if (n == MM_SP) mma_stage<P, NT, true, BIL, GF>(st, n, a.rowb, doff, acc, F);         \
-            else mma_stage<P, NT, false, BIL, GF>(st, n, a.rowb, doff, acc, F);                   \
-            it++;                                                                                 \
-            if (++cslot == a.nst) {                                                               \
-                cslot = 0;                                                                        \
-                cphase ^= 1;                                                                      \
-            }                                                                                     \
-            __syncwarp(); /* every lane has read the slot */                                      \
-            issue();                                                                              \
-        }                                                                                         \
+        const int nmine = (sb - sa - warp + MM_WARPS - 1) / MM_WARPS;
+#define DGV_MMA_CASE(NT)                                                                              \
+    case NT:                                                                                          \
+        for (int s = 0; s < nmine; s++) {                                                             \
+            int n = 0;                                                                                \
+            if (!fetch.wait(a, n)) break;                                                             \
+            if (n == MM_SP) mma_stage<P, NT, true, BIL, GF>(fetch.stage(a), n, a.rowb, doff, acc, F); \
+            else mma_stage<P, NT, false, BIL, GF>(fetch.stage(a), n, a.rowb, doff, acc, F);           \
+            fetch.done(a);                                                                            \
+        }                                                                                             \
         break;
         switch (nt) {
             DGV_MMA_CASE(1)
@@ -392,9 +424,175 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_collide_mma(const __grid_cons
         double *out = a.partial + ((size_t)vdf * a.nchunks + chunk) * ((size_t)a.ncell * P);
         for (int i = threadIdx.x; i < a.ncell * P; i += MM_THREADS) out[i] = part[i];
     }
-    // after a wait that gave up: let the copies already issued land
-    if (!ok)
-        for (; it < issued; it++) mbar_wait(&full[it % a.nst], (it / a.nst) & 1, a.err, a.wait_ns);
+    fetch.drain(a);
+}
+
+// ----------------------------------------------------------------------------
+// FP32-compensated Q on the same units.  The arithmetic is that of the
+// lane-wise kernel, sum for sum: FP32 products f(a) f(b), the 16-pair groups of
+// a block summed by FP32 multiply-adds in pair order, group sums added with
+// two-sum into (sum, correction); only the order of the group sums differs.
+// A stage is one group.  The warp's 32 lanes are 4 column groups x 8 row
+// groups: lane (pg, rg) keeps the sums of rows rg + 8j (j < A) and columns
+// PB pg .. PB pg + PB - 1 (PB = ceil(P/4)), so that a pair costs it PB values
+// and A products from shared memory or other lanes for A * PB multiply-adds:
+// shared memory delivers one word per lane and cycle to one warp of the SM,
+// which bounds a kernel with one row and all P columns per lane (32 words for
+// 27 multiply-adds).  A product is formed by one of the four lanes that need
+// it and handed on by shuffles.
+// Measured (B200): a stage of 64 rows takes 724 SM cycles, 216 of them
+// multiply-adds; shared memory's and the shuffles' ~21 words per pair and
+// their latency bound it (two rows and all columns per lane: 655, but rows in
+// steps of 32; 12 or 16 warps of 32 rows: 405 per 32 rows).  Per Q at 21^3 with
+// projection, one cell per lane -> this kernel: 18.3 -> 3.8 ms.
+constexpr int FC_WARPS = 8, FC_THREADS = 32 * FC_WARPS;
+constexpr int FC_TILE = 16, FC_MT = 4;  // rows per tile (A = 2 per tile); tiles per unit
+
+template <bool GF>
+struct F32F {
+    uint32_t f_s;
+    const float *f;
+    __device__ __forceinline__ int scaled(int o) const { return GF ? o : 4 * o; }
+    __device__ __forceinline__ float fat(int q) const
+    {
+        if constexpr (GF) {
+            return __ldg(f + q);
+        } else {
+            float x;
+            asm("ld.shared.f32 %0, [%1];" : "=f"(x) : "r"(f_s + q));
+            return x;
+        }
+    }
+};
+
+// the n pairs of one group added into (sum, correction); d1, d2: places of the
+// cells whose products this lane forms (rows rg + 8 pg and rg + 8 pg + 32)
+template <int P, int A, bool GF>
+__device__ __forceinline__ void f32_stage(const unsigned char *st, int n, int d1, int d2, float (*sm)[(P + 3) / 4],
+                                          float (*cr)[(P + 3) / 4], const F32F<GF> &F)
+{
+    constexpr int RB = ((2 + P) + 3) / 4 * 16;  // bytes of a row: offsets, values, zeros
+    constexpr int PB = (P + 3) / 4;
+    const int pg = threadIdx.x & 3;
+    float part[A][PB];
+#pragma unroll
+    for (int j = 0; j < A; j++)
+#pragma unroll
+        for (int i = 0; i < PB; i++) part[j][i] = 0.f;
+#pragma unroll 4
+    for (int k = 0; k < n; k++) {
+        const int2 o = *reinterpret_cast<const int2 *>(st + k * RB);
+        const float *row = reinterpret_cast<const float *>(st + k * RB) + 2 + PB * pg;
+        const int a1 = F.scaled(o.x), a2 = F.scaled(o.y);
+        const float x1 = F.fat(a1 + d1) * F.fat(a2 + d1);
+        const float x2 = A > 4 ? F.fat(a1 + d2) * F.fat(a2 + d2) : 0.f;
+        float v[PB];
+#pragma unroll
+        for (int i = 0; i < PB; i++) v[i] = row[i];
+#pragma unroll
+        for (int j = 0; j < A; j++) {
+            const float x = __shfl_sync(0xffffffffu, j < 4 ? x1 : x2, j & 3, 4);
+#pragma unroll
+            for (int i = 0; i < PB; i++) part[j][i] = fmaf(v[i], x, part[j][i]);
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < A; j++)
+#pragma unroll
+        for (int i = 0; i < PB; i++) {  // two-sum: sum + correction carries the group sum exactly
+            const float x = part[j][i], s = sm[j][i], t = s + x, bp = t - s;
+            cr[j][i] += (s - (t - bp)) + (x - bp);
+            sm[j][i] = t;
+        }
+}
+
+template <int P, bool GF>
+__global__ void __launch_bounds__(FC_THREADS, 1) k_collide_f32(const __grid_constant__ MmaArgs a)
+{
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ int rowcell[FC_TILE * FC_MT];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int vdf = blockIdx.x, chunk = blockIdx.y, pg = lane & 3, rg = lane >> 2;
+    constexpr int PB = (P + 3) / 4, CW = 4 * PB;
+    float *f_s = reinterpret_cast<float *>(smem + a.off_f);
+    double *red = reinterpret_cast<double *>(smem + a.off_red);  // [FC_WARPS][8][CW]
+    double *part = a.part_smem ? reinterpret_cast<double *>(smem + a.off_part)
+                               : a.partial + ((size_t)vdf * a.nchunks + chunk) * ((size_t)a.ncell * P);
+    MmaFetch<FC_WARPS> fetch(a, smem, warp, a.bounds[chunk], a.bounds[chunk + 1]);
+    if constexpr (!GF) {
+        const double *f = a.f + (size_t)vdf * a.N;
+        for (int i = threadIdx.x; i < (int)a.N; i += FC_THREADS) {
+            const int cell = i / P, l = i - cell * P;
+            f_s[l * a.Nc + cell] = (float)__ldg(f + i);
+        }
+    }
+    for (int i = threadIdx.x; i < a.ncell * P; i += FC_THREADS) part[i] = 0.0;
+    __syncthreads();
+    F32F<GF> F;
+    F.f_s = smem_u32(f_s);
+    F.f = GF ? reinterpret_cast<const float *>(a.fg) + (size_t)vdf * a.N : nullptr;
+
+    for (int u = fetch.b0.x; u <= fetch.b1.x; u++) {
+        const MmaUnit un = a.units[u];
+        const int sa = u == fetch.b0.x ? fetch.b0.y : un.stage0, sb = u == fetch.b1.x ? fetch.b1.y : un.stage1;
+        if (sa >= sb) continue;  // the same in every warp
+        const int nt = (un.nrow + FC_TILE - 1) / FC_TILE;
+        // rows past the last repeat it (they are not stored)
+        const int d1 = F.scaled(mma_cell(un, un.row0 + min(rg + 8 * pg, un.nrow - 1), a.Mv, a.Mw));
+        const int d2 = F.scaled(mma_cell(un, un.row0 + min(rg + 8 * pg + 32, un.nrow - 1), a.Mv, a.Mw));
+        if (warp < 2) {
+            const int r = 32 * warp + lane;
+            rowcell[r] = mma_cell(un, un.row0 + min(r, un.nrow - 1), a.Mv, a.Mw) - a.cell0;
+        }
+        float sm[2 * FC_MT][PB], cr[2 * FC_MT][PB];
+#pragma unroll
+        for (int j = 0; j < 2 * FC_MT; j++)
+#pragma unroll
+            for (int i = 0; i < PB; i++) sm[j][i] = cr[j][i] = 0.f;
+        const int nmine = (sb - sa - warp + FC_WARPS - 1) / FC_WARPS;
+#define DGV_F32_CASE(NT)                                                    \
+    case NT:                                                                \
+        for (int s = 0; s < nmine; s++) {                                   \
+            int n = 0;                                                      \
+            if (!fetch.wait(a, n)) break;                                   \
+            f32_stage<P, 2 * NT, GF>(fetch.stage(a), n, d1, d2, sm, cr, F); \
+            fetch.done(a);                                                  \
+        }                                                                   \
+        break;
+        switch (nt) {
+            DGV_F32_CASE(1)
+            DGV_F32_CASE(2)
+            DGV_F32_CASE(3)
+            DGV_F32_CASE(4)
+        }
+#undef DGV_F32_CASE
+        // the warps' sums in FP64, eight rows at a time, in warp order, into
+        // the CTA's partial Q
+#pragma unroll
+        for (int j = 0; j < 2 * FC_MT; j++) {
+            if (8 * j >= un.nrow) break;
+            const int row = threadIdx.x / P, p = threadIdx.x - row * P;
+            const bool mine = row < 8 && 8 * j + row < un.nrow;
+#pragma unroll
+            for (int i = 0; i < PB; i++)
+                red[(size_t)(warp * 8 + rg) * CW + PB * pg + i] = (double)sm[j][i] + (double)cr[j][i];
+            __syncthreads();
+            if (mine) {
+                double *dst = part + (size_t)rowcell[8 * j + row] * P + p;
+                const double old = *dst;
+                double s = 0.0;
+#pragma unroll
+                for (int w = 0; w < FC_WARPS; w++) s += red[(size_t)(w * 8 + row) * CW + p];
+                *dst = old + s;
+            }
+            __syncthreads();
+        }
+    }
+    if (a.part_smem) {
+        double *out = a.partial + ((size_t)vdf * a.nchunks + chunk) * ((size_t)a.ncell * P);
+        for (int i = threadIdx.x; i < a.ncell * P; i += FC_THREADS) out[i] = part[i];
+    }
+    fetch.drain(a);
 }
 
 // q[v][i] = scale * (2 * sum_chunks partial[v][chunk][i]) / w[cell0*P + i]:
@@ -426,10 +624,10 @@ __global__ void __launch_bounds__(256) k_reduce_partials(const double *partial, 
 // ----------------------------------------------------------------------------
 // The stage list of the layout (blocks sorted by box) and, per range of output
 // cells, the units: built on first use and kept with the A-arrays.
-static int mma_boxes(Ctx *c)
+static int mma_boxes(Ctx *c, MmaList &M, bool across)
 {
-    Layout &L = c->lay;
-    if (L.mma_segs) return DGV_OK;
+    const Layout &L = c->lay;
+    if (M.segs) return DGV_OK;
     std::vector<int> order(L.nblocks);
     std::iota(order.begin(), order.end(), 0);
     auto key = [&](int b) {
@@ -441,13 +639,13 @@ static int mma_boxes(Ctx *c)
     std::vector<unsigned long long> keys(L.nblocks);
     for (long long b = 0; b < L.nblocks; b++) keys[b] = key((int)b);
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return keys[x] < keys[y]; });
-    // a box's pairs in block order, cut into stages of MM_SP; a stage's pairs
-    // come from one block or from several, a segment for each
+    // a box's pairs in block order, cut into stages of MM_SP: across blocks (a
+    // segment for each block a stage draws on), or anew from each block's start
     std::vector<unsigned long long> seg;
     std::vector<int> sfirst;
     seg.reserve((size_t)(L.npairs / MM_SP + 2 * L.nblocks + 1));
     sfirst.reserve((size_t)(L.npairs / MM_SP + L.nblocks + 2));
-    L.mma_box.clear();
+    M.box.clear();
     int room = 0;  // pairs the open stage still takes
     for (long long i = 0; i < L.nblocks; i++) {
         const BlockInfo &bi = L.h_blk[order[i]];
@@ -455,9 +653,10 @@ static int mma_boxes(Ctx *c)
             MmaBox bx;
             for (int d = 0; d < 3; d++) { bx.lo[d] = bi.lo[d]; bx.hi[d] = bi.hi[d]; }
             bx.stage0 = (long long)sfirst.size();
-            L.mma_box.push_back(bx);
+            M.box.push_back(bx);
             room = 0;
         }
+        if (!across) room = 0;
         for (int o = 0; o < bi.count;) {
             if (room == 0) {
                 sfirst.push_back((int)seg.size());
@@ -469,7 +668,7 @@ static int mma_boxes(Ctx *c)
             room -= n;
             o += n;
         }
-        L.mma_box.back().stage1 = (long long)sfirst.size();
+        M.box.back().stage1 = (long long)sfirst.size();
     }
     if (seg.size() > (size_t)INT32_MAX) return set_err(c, DGV_EUNSUP, "collide: too many pairs for the stage list");
     sfirst.push_back((int)seg.size());
@@ -485,26 +684,28 @@ static int mma_boxes(Ctx *c)
         return set_err(c, rc == cudaErrorMemoryAllocation ? DGV_ENOMEM : DGV_ECUDA,
                        std::string("collide: stage list: ") + cudaGetErrorString(rc));
     }
-    L.mma_segs = d;
-    L.mma_sfirst = e;
+    M.segs = d;
+    M.sfirst = e;
     return DGV_OK;
 }
 
 // Units of the boxes' cells in [cell0, cell1) (contiguous in a box's node
-// order), tiles spread evenly over a box's units.
-static int mma_plan(Ctx *c, int cell0, int cell1, MmaPlan **out)
+// order), tiles of `rows` cells spread evenly over a box's units.
+struct MmaShape {
+    int rows, tiles;                       // rows per tile, tiles per unit at most
+    int c_tile, c_stage, c_unit, c_flush;  // costs (SM cycles, fitted): stage per tile, stage, unit, its end per tile
+};
+
+static int mma_plan(Ctx *c, MmaList &M, const MmaShape &S, int cell0, int cell1, MmaPlan **out)
 {
-    Layout &L = c->lay;
     const Grid &g = c->grid;
-    int rc = mma_boxes(c);
-    if (rc) return rc;
     const std::pair<int, int> key(cell0, cell1);
-    auto it = L.mma_plans.find(key);
-    if (it != L.mma_plans.end()) { *out = &it->second; return DGV_OK; }
+    auto it = M.plans.find(key);
+    if (it != M.plans.end()) { *out = &it->second; return DGV_OK; }
     std::vector<MmaUnit> units;
     MmaPlan pl;
     pl.cost.push_back(0);
-    for (const MmaBox &bx : L.mma_box) {
+    for (const MmaBox &bx : M.box) {
         const int len[3] = {bx.hi[0] - bx.lo[0] + 1, bx.hi[1] - bx.lo[1] + 1, bx.hi[2] - bx.lo[2] + 1};
         if (len[0] <= 0 || len[1] <= 0 || len[2] <= 0) continue;
         // rows of the box whose cell lies before `cell`
@@ -519,7 +720,7 @@ static int mma_plan(Ctx *c, int cell0, int cell1, MmaPlan **out)
         };
         const int whole = len[0] * len[1] * len[2];
         const int r0 = cell0 > 0 ? before(cell0) : 0, r1 = cell1 < g.Nc ? before(cell1) : whole;
-        const int tiles = (r1 - r0 + 7) / 8, nu = (tiles + MM_MT - 1) / MM_MT;
+        const int tiles = (r1 - r0 + S.rows - 1) / S.rows, nu = (tiles + S.tiles - 1) / S.tiles;
         int t0 = 0;
         for (int k = 0; k < nu; k++) {
             const int t1 = (int)((long long)tiles * (k + 1) / nu);
@@ -527,15 +728,13 @@ static int mma_plan(Ctx *c, int cell0, int cell1, MmaPlan **out)
             std::memset(&un, 0, sizeof(un));
             un.stage0 = (int)bx.stage0;
             un.stage1 = (int)bx.stage1;
-            un.row0 = r0 + 8 * t0;
-            un.nrow = std::min(8 * (t1 - t0), r1 - un.row0);
+            un.row0 = r0 + S.rows * t0;
+            un.nrow = std::min(S.rows * (t1 - t0), r1 - un.row0);
             for (int d = 0; d < 3; d++) { un.lo[d] = (signed char)bx.lo[d]; un.len[d] = (signed char)len[d]; }
             units.push_back(un);
-            // SM cycles of a stage of t tiles and of the end of a unit, as
-            // measured per CTA range and fitted (see MmaPlan)
-            pl.per_stage.push_back(MM_C_TILE * (t1 - t0) + MM_C_STAGE);
-            pl.per_unit.push_back(MM_C_UNIT + MM_C_FLUSH * (t1 - t0));
-            pl.cost.push_back(pl.cost.back() + (long long)pl.per_stage.back() * (un.stage1 - un.stage0) + pl.per_unit.back());
+            pl.per_stage.push_back(S.c_tile * (t1 - t0) + S.c_stage);
+            pl.cost.push_back(pl.cost.back() + (long long)pl.per_stage.back() * (un.stage1 - un.stage0) + S.c_unit +
+                              S.c_flush * (t1 - t0));
             pl.first.push_back(un.stage0);
             pl.last.push_back(un.stage1);
             t0 = t1;
@@ -548,7 +747,7 @@ static int mma_plan(Ctx *c, int cell0, int cell1, MmaPlan **out)
         cudaFree(pl.units);
         return set_err(c, DGV_ECUDA, std::string("collide plan: ") + cudaGetErrorString(e));
     }
-    *out = &(L.mma_plans[key] = std::move(pl));
+    *out = &(M.plans[key] = std::move(pl));
     return DGV_OK;
 }
 
@@ -583,11 +782,11 @@ static int mma_bounds(Ctx *c, MmaPlan *pl, int nchunks, const int2 **out)
 // Ranges per VDF: the smallest count whose CTAs fill the last wave to 99.5 % (one
 // CTA per SM, all of equal cost), else the one that fills it best, with at
 // least four stages per warp and at most four waves.
-static int mma_chunks(int nsm, int nvdf, long long stages)
+static int mma_chunks(int nsm, int nvdf, int warps, long long stages)
 {
     int best = 1;
     double eff = 0.0;
-    const int most = (int)std::max<long long>(1, std::min<long long>((4LL * nsm + nvdf - 1) / nvdf, stages / (4 * MM_WARPS)));
+    const int most = (int)std::max<long long>(1, std::min<long long>((4LL * nsm + nvdf - 1) / nvdf, stages / (4 * warps)));
     for (int k = 1; k <= most; k++) {
         const long long ctas = (long long)nvdf * k, waves = (ctas + nsm - 1) / nsm;
         const double e = (double)ctas / (double)(waves * nsm);
@@ -600,36 +799,47 @@ static int mma_chunks(int nsm, int nvdf, long long stages)
 typedef void (*MmaFn)(const MmaArgs);
 
 template <int P>
-static MmaFn mma_pick(bool bil, bool gf)
+static MmaFn mma_pick(bool f32, bool bil, bool gf)
 {
+    if (f32) return gf ? k_collide_f32<P, true> : k_collide_f32<P, false>;
     if (bil) return gf ? k_collide_mma<P, true, true> : k_collide_mma<P, true, false>;
     return gf ? k_collide_mma<P, false, true> : k_collide_mma<P, false, false>;
 }
 
 bool mma_serves(const Ctx *c) { return c->grid.P == 27 || c->grid.P == 8; }
 
-int collide_mma_device(Ctx *c, const double *d_f, const double *d_g, double *d_q, int nvdf, double scale, int cell0,
-                       int cell1)
+// Q(f,f) in FP64 or FP32-compensated arithmetic, or with d_g the mixed terms
+// of f and g in FP64, on the output cells [cell0, cell1)
+int collide_mma_device(Ctx *c, const double *d_f, const double *d_g, double *d_q, int nvdf, int precision, double scale,
+                       int cell0, int cell1)
 {
     const Grid &g = c->grid;
     Layout &L = c->lay;
+    const bool bil = d_g != nullptr, f32 = precision == DGV_PREC_F32C;
     int maxsm = 0, nsm = 148;
     DGV_CUDA(c, cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
     DGV_CUDA(c, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
     if (g.N > INT32_MAX / 2) return set_err(c, DGV_EUNSUP, "collide: grid too large");  // gather indices are ints
+    int rc;
+    if (f32 && (rc = ensure_rows32(c))) return rc;  // rebuilt if released
+    // costs fitted to the measured cycles of the ranges at 15^3, 21^3 and 27^3
+    const MmaShape S = f32 ? MmaShape{FC_TILE, FC_MT, 125, 235, 3000, 1500} : MmaShape{8, MM_MT, 66, 80, 3000, 600};
+    MmaList &M = f32 ? L.groups : L.mma;
     MmaPlan *pl = nullptr;
-    int rc = mma_plan(c, cell0, cell1, &pl);
-    if (rc) return rc;
-    const bool bil = d_g != nullptr;
+    if ((rc = mma_boxes(c, M, !f32))) return rc;
+    if ((rc = mma_plan(c, M, S, cell0, cell1, &pl))) return rc;
     MmaArgs a;
     std::memset(&a, 0, sizeof(a));
-    a.rowb = L.RD64 * 8;
-    const int stage = MM_WARPS * MM_SP * a.rowb;  // one ring stage of every warp
-    const int fb = (int)std::min<long long>((g.N * 8 + 15) / 16 * 16, 1 << 28), nf = bil ? 2 : 1;
-    const int red = MM_WARPS * 8 * ((g.P + 7) / 8 * 8) * 8, tail = red + MM_WARPS * MM_MAXST * 12 + 16 + 8 * MM_MT * 4;
+    a.rowb = f32 ? L.RW32 * 4 : L.RD64 * 8;
+    const int warps = f32 ? FC_WARPS : MM_WARPS;
+    const int stage = warps * MM_SP * a.rowb;  // one ring stage of every warp
+    const int nf = bil ? 2 : 1, fb = (int)std::min<long long>((g.N * (f32 ? 4 : 8) + 15) / 16 * 16, 1 << 28);
+    // a tile's sums of every warp at a unit's end
+    const int red = warps * 8 * (f32 ? (g.P + 3) / 4 * 4 : (g.P + 7) / 8 * 8) * 8;
+    const int tail = red + warps * MM_MAXST * 12 + 16 + 8 * MM_MT * 4;
     // at least two stages beside the shared copies, else f from global memory;
-    // what room is left goes to the partial Q, then to up to four tiles at a
-    // time at a unit's end, then to more stages
+    // what room is left goes to the partial Q, then (FP64) to up to four tiles
+    // at a time at a unit's end, then to more stages
     const bool gf = c->f_global == 1 || (long long)nf * fb + tail + 2 * stage > maxsm;
     int room = maxsm - tail - (gf ? 0 : nf * fb) - 2 * stage;
     if (room < 0) return set_err(c, DGV_EUNSUP, "collide: the row ring does not fit in shared memory");
@@ -638,7 +848,7 @@ int collide_mma_device(Ctx *c, const double *d_f, const double *d_g, double *d_q
     a.part_smem = pb > 0 && pb <= room;
     if (a.part_smem) room -= pb;
     a.red_tiles = 1;
-    while (a.part_smem && a.red_tiles < 4 && room >= a.red_tiles * red) {
+    while (!f32 && a.part_smem && a.red_tiles < 4 && room >= a.red_tiles * red) {
         room -= a.red_tiles * red;
         a.red_tiles *= 2;
     }
@@ -648,29 +858,30 @@ int collide_mma_device(Ctx *c, const double *d_f, const double *d_g, double *d_q
     a.off_part = a.off_f + (gf ? 0 : nf * fb);
     a.off_red = a.off_part + (a.part_smem ? pb : 0);
     a.off_bar = a.off_red + a.red_tiles * red;
-    const size_t smem = (size_t)a.off_bar + MM_WARPS * MM_MAXST * 12;
-    int nchunks = c->nchunks_opt > 0 ? std::min<long long>(c->nchunks_opt, std::max<long long>(1, L.nblocks))
-                                     : mma_chunks(nsm, nvdf, pl->cost.back() / (MM_C_TILE * MM_MT + MM_C_STAGE));
+    const size_t smem = (size_t)a.off_bar + warps * MM_MAXST * 12;
+    const int nchunks = c->nchunks_opt > 0 ? (int)std::min<long long>(c->nchunks_opt, std::max<long long>(1, L.nblocks))
+                                           : mma_chunks(nsm, nvdf, warps, pl->cost.back() / (S.c_tile * S.tiles + S.c_stage));
     const int2 *bounds = nullptr;
     if ((rc = mma_bounds(c, pl, nchunks, &bounds))) return rc;
     if ((rc = ensure_buffer(c, &c->d_partial, &c->partial_bytes, (size_t)nvdf * nchunks * len * sizeof(double)))) return rc;
     if ((rc = ensure_errflag(c))) return rc;
     if (gf) {
         const void *p = nullptr;
-        if ((rc = f_local_major(c, d_f, d_g, nvdf, false, &p))) return rc;
+        if ((rc = f_local_major(c, d_f, d_g, nvdf, f32, &p))) return rc;
         a.fg = static_cast<const double *>(p);
         a.gg = bil ? a.fg + (size_t)nvdf * g.N : nullptr;
     }
-    a.f = d_f; a.g = d_g; a.partial = c->d_partial; a.rows = (const char *)L.rows64;
-    a.segs = (const unsigned long long *)L.mma_segs; a.sfirst = (const int *)L.mma_sfirst; a.units = (const MmaUnit *)pl->units; a.bounds = bounds;
+    a.f = d_f; a.g = d_g; a.partial = c->d_partial; a.rows = (const char *)(f32 ? L.rows32 : L.rows64);
+    a.segs = (const unsigned long long *)M.segs; a.sfirst = (const int *)M.sfirst;
+    a.units = (const MmaUnit *)pl->units; a.bounds = bounds;
     a.err = c->d_err; a.N = g.N; a.Nc = g.Nc; a.Mv = g.d.Mv; a.Mw = g.d.Mw; a.nchunks = nchunks;
     a.cell0 = cell0; a.ncell = cell1 - cell0; a.wait_ns = wait_limit_ns(c);
-    MmaFn fn = g.P == 27 ? mma_pick<27>(bil, gf) : mma_pick<8>(bil, gf);
+    MmaFn fn = g.P == 27 ? mma_pick<27>(f32, bil, gf) : mma_pick<8>(f32, bil, gf);
     DGV_CUDA(c, cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     KTimer kt(c);
     if (pl->nunits > 0) {
         // VDF fastest: the CTAs resident at one time read the same rows
-        fn<<<dim3(nvdf, nchunks), MM_THREADS, smem, c->stream>>>(a);
+        fn<<<dim3(nvdf, nchunks), 32 * warps, smem, c->stream>>>(a);
         DGV_CUDA(c, cudaGetLastError());
     } else {
         DGV_CUDA(c, cudaMemsetAsync(c->d_partial, 0, (size_t)nvdf * nchunks * len * sizeof(double), c->stream));

@@ -52,14 +52,22 @@ struct MmaBox {
 };
 
 // The units of a range of output cells (collide_mma.cu): device array, and per
-// unit the running cost, first stage and cost per stage; per number of ranges
+// unit the running cost, stage range and cost per stage; per number of ranges
 // the device array of their bounds
 struct MmaPlan {
     void *units = nullptr;
     int nunits = 0;
     std::vector<long long> cost;
-    std::vector<int> first, last, per_stage, per_unit;
+    std::vector<int> first, last, per_stage;
     std::map<int, void *> bounds;
+};
+
+// Stages of the layout's pairs in box order (collide_mma.cu; device arrays),
+// the boxes and the plans per range of output cells.  Built on first use.
+struct MmaList {
+    void *segs = nullptr, *sfirst = nullptr;
+    std::vector<MmaBox> box;
+    std::map<std::pair<int, int>, MmaPlan> plans;
 };
 
 // Device copy of the A-arrays in the pair layout.
@@ -80,11 +88,9 @@ struct Layout {
     std::vector<double> h_work;       // per block: pairs x valid shifts
     // work partitions: nchunks -> device array of nchunks+1 block bounds
     std::map<int, int *> chunks;
-    // FP64 tensor instructions (built on first use): stages in box order, the
-    // boxes, and the units per range of output cells
-    void *mma_segs = nullptr, *mma_sfirst = nullptr;  // device
-    std::vector<MmaBox> mma_box;
-    std::map<std::pair<int, int>, MmaPlan> mma_plans;
+    // boxes (collide_mma.cu): stages that run on across blocks (FP64), and
+    // stages that are the 16-pair groups of one block (FP32-compensated)
+    MmaList mma, groups;
     // tensor-core form (built on first use): per block ceil(count/64) chunk
     // records of split-fp16 value tiles, their first record per block, the
     // power-of-two value scale, and the block sets of one launch each
@@ -245,8 +251,8 @@ int get_chunks(Ctx *c, int nchunks, int **d_bounds);
 int collide_device(Ctx *c, const double *d_f, double *d_q, int nvdf, int precision,
                    double scale);
 bool mma_serves(const Ctx *c);
-int collide_mma_device(Ctx *c, const double *d_f, const double *d_g, double *d_q, int nvdf, double scale, int cell0,
-                       int cell1);
+int collide_mma_device(Ctx *c, const double *d_f, const double *d_g, double *d_q, int nvdf, int precision, double scale,
+                       int cell0, int cell1);
 int collide_tc_device(Ctx *c, const double *d_f, double *d_q, int nvdf, double scale);
 int collide_cells_device(Ctx *c, const double *d_f, double *d_q, int nvdf, int precision, int cell0, int cell1);
 int jvp_device(Ctx *c, const double *d_f, const double *d_df, double *d_q, int precision);

@@ -26,11 +26,13 @@ void free_layout(Layout &L)
     if (L.rows64) cudaFree(L.rows64);
     if (L.rows32) cudaFree(L.rows32);
     for (auto &kv : L.chunks) cudaFree(kv.second);
-    if (L.mma_segs) cudaFree(L.mma_segs);
-    if (L.mma_sfirst) cudaFree(L.mma_sfirst);
-    for (auto &kv : L.mma_plans) {
-        if (kv.second.units) cudaFree(kv.second.units);
-        for (auto &b : kv.second.bounds) cudaFree(b.second);
+    for (MmaList *m : {&L.mma, &L.groups}) {
+        if (m->segs) cudaFree(m->segs);
+        if (m->sfirst) cudaFree(m->sfirst);
+        for (auto &kv : m->plans) {
+            if (kv.second.units) cudaFree(kv.second.units);
+            for (auto &b : kv.second.bounds) cudaFree(b.second);
+        }
     }
     if (L.tc_V) cudaFree(L.tc_V);
     if (L.tc_chunk_start) cudaFree(L.tc_chunk_start);

@@ -98,3 +98,28 @@ def test_non_finite_values_stay_where_they_belong():
         assert np.abs(q[ok] - ref[ok]).max() < TOL * np.abs(ref[ok]).max() if ok.any() else True
     finally:
         s.close()
+
+
+@pytest.mark.parametrize("g", GRIDS, ids=lambda g: "x".join(str(v) for v in g.values()))
+def test_fp32_compensated_on_the_same_units(g):
+    """FP32 products in groups of 16 pairs, compensated: within the 1e-6 of the
+    arithmetic from FP64, and the same up to the order of the compensated group
+    sums (a few 2^-48) whatever the ranges, slices or the place of f."""
+    s = _solver(g)
+    try:
+        f = _vdfs(s, 3)
+        ref = _lanewise(s, f)
+        q = s.EvalCollisionPeriodicAPlus_DGV(f, precision="f32c")
+        assert rel_err(q, ref) < 1e-6
+        for chunks in (1, 7, 300):
+            s.set_nchunks(chunks)
+            assert rel_err(s.EvalCollisionPeriodicAPlus_DGV(f, precision="f32c"), q) < 1e-11
+        s.set_nchunks(0)
+        s.set_f_global(True)
+        assert np.array_equal(s.EvalCollisionPeriodicAPlus_DGV(f, precision="f32c"), q)
+        s.set_f_global(False)
+        cuts = sorted({0, s.Nc // 3, s.Nc})
+        parts = [s.collide_cells(f, a, b, precision="f32c") for a, b in zip(cuts, cuts[1:])]
+        assert rel_err(np.concatenate(parts, axis=-1), q) < 1e-11
+    finally:
+        s.close()
