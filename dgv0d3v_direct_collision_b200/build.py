@@ -31,6 +31,7 @@ SOURCES = [
     ("collide_mma.cu", []),
     ("collide_tc.cu", []),
     ("adjoint.cu", []),
+    ("adjoint_mma.cu", []),
     ("noalloc.cu", []),
     ("synth.cu", ["-fmad=false"]),
     ("seta.cu", ["-fmad=false"]),

@@ -175,10 +175,8 @@ int vjp_device(Ctx *c, const double *d_f, const double *d_v, double *d_g, int pr
 #define DGV_VJP_PICK(...) fn = gf ? k_vjp_pipe<__VA_ARGS__, true> : k_vjp_pipe<__VA_ARGS__, false>
     switch (g.P) {
     case 1: DGV_VJP_PICK(1, false); break;
-    case 8: DGV_VJP_PICK(8, false); break;
-    case 27: DGV_VJP_PICK(27, false); break;
     case 125: DGV_VJP_PICK(25, true); break;  // slices of 25 basis functions per CTA
-    default: return set_err(c, DGV_EUNSUP, "vjp: this build supports 1, 8, 27 or 125 nodes per cell");
+    default: return set_err(c, DGV_EUNSUP, "vjp: this build supports 1, 8, 27 or 125 nodes per cell");  // 8, 27: adjoint_mma.cu
     }
 #undef DGV_VJP_PICK
     const size_t ring = std::min<size_t>(64 * 1024, (size_t)maxsm - fbytes - tail);

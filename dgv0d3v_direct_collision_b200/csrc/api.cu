@@ -760,6 +760,8 @@ int dgv_vjp_batched(dgv_ctx *ctx, int32_t nb, const double *f, const double *v, 
     TRY(out_ptr(c, g, n, &dg, &host));
     if (precision == DGV_PREC_TC) {
         TRY(vjp_tc_device(c, d1, d2, dg, nb));
+    } else if (mma_serves(c)) {
+        TRY(vjp_mma_device(c, d1, d2, dg, nb));
     } else {
         for (int32_t b = 0; b < nb; b++) TRY(vjp_device(c, d1 + b * N, d2 + b * N, dg + b * N, precision));
     }

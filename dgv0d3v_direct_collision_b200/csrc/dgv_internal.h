@@ -91,6 +91,10 @@ struct Layout {
     // boxes (collide_mma.cu): stages that run on across blocks (FP64), and
     // stages that are the 16-pair groups of one block (FP32-compensated)
     MmaList mma, groups;
+    // FP64 adjoint (adjoint_mma.cu; built on first use): pair tiles per block
+    // and work items, device arrays
+    void *vjp_first = nullptr, *vjp_tiles = nullptr, *vjp_items = nullptr;
+    long long vjp_nitems = 0;
     // tensor-core form (built on first use): per block ceil(count/64) chunk
     // records of split-fp16 value tiles, their first record per block, the
     // power-of-two value scale, and the block sets of one launch each
@@ -149,7 +153,8 @@ struct Ctx {
     // CUDA-core kernels with f in global memory: local-major copies f[v][l*Nc + cell]
     double *d_fg = nullptr;
     size_t fg_bytes = 0;
-    // VJP: local-major accumulator g_lm[l*Nc + cell]
+    // VJP: local-major accumulator g_lm[l*Nc + cell], or the sums, the
+    // item counter and c = 2v/w (adjoint_mma.cu)
     double *d_glm = nullptr;
     size_t glm_bytes = 0;
     // Adams-Bashforth history: right sides frhs1..frhs5 (newest first)
@@ -257,6 +262,7 @@ int collide_tc_device(Ctx *c, const double *d_f, double *d_q, int nvdf, double s
 int collide_cells_device(Ctx *c, const double *d_f, double *d_q, int nvdf, int precision, int cell0, int cell1);
 int jvp_device(Ctx *c, const double *d_f, const double *d_df, double *d_q, int precision);
 int vjp_device(Ctx *c, const double *d_f, const double *d_v, double *d_g, int precision);
+int vjp_mma_device(Ctx *c, const double *d_f, const double *d_v, double *d_g, int nvdf);
 int vjp_tc_device(Ctx *c, const double *d_f, const double *d_v, double *d_g, int nvdf);
 int moments_device(Ctx *c, const double *d_f, int nvdf, double *h_out);
 int project_device(Ctx *c, double *d_q, int nvdf);

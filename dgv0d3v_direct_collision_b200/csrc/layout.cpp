@@ -34,6 +34,8 @@ void free_layout(Layout &L)
             for (auto &b : kv.second.bounds) cudaFree(b.second);
         }
     }
+    for (void *p : {L.vjp_first, L.vjp_tiles, L.vjp_items})
+        if (p) cudaFree(p);
     if (L.tc_V) cudaFree(L.tc_V);
     if (L.tc_chunk_start) cudaFree(L.tc_chunk_start);
     if (L.tc2_W) cudaFree(L.tc2_W);
