@@ -8,18 +8,24 @@
 //   g(c1+D, l1) += sum_l2 vA[D, k] f(c2+D, l2)
 //   g(c2+D, l2) += sum_l1 vA[D, k] f(c1+D, l1).
 // One cell per lane and two atomics per pair and cell (adjoint.cu) is bound by
-// the atomics.  Here a warp takes a block and up to 24 of its cells (rows) at a
+// the atomics.  Here a warp takes a block and up to 16 of its cells (rows) at a
 // time, keeps their c as A fragments in registers, and multiplies them with
 // tiles of up to 8 pairs of one l1 (mma.m8n8k4, K = P padded to a multiple of
-// 4); both scatters stay inside the warp: the sums over l2 in registers until
-// the l1 ends, those over l1 in shared memory.  At the end of the block 2 P
-// atomics per cell go to g, 27 consecutive doubles per row, instead of two per
-// pair: 54 instead of ~745 at 27^3.  As before the order of the atomics, and so
-// the last bits of g, vary from run to run.
+// 4).  Both scatters stay inside the warp: the sums over l2 in registers until
+// the l1 ends, those over l1 in shared memory until the block ends, so that at
+// most 2 P atomics per cell go to g, 54 instead of ~745 at 27^3.  As before the
+// order of the atomics, and so the last bits of g, vary from run to run.
 //
-// Warps are independent (no CTA barrier after the start): each takes the next
-// item, heaviest blocks first, from a counter, and streams the block's rows
-// through a ring of bulk copies of its own.
+// Warps are independent (no CTA barrier): each takes the next item, heaviest
+// blocks first, from a counter, and streams the block's rows through a ring of
+// bulk copies of its own.
+//
+// Measured (B200, 1965 MHz), one VDF at 21^3: 44.9 ms with one cell per lane,
+// 5.6 ms here.  The products take 2.4 ms of that (76 % of a tile's pairs are
+// real: a block has ~16 pairs per l1); shared memory delivers 63 % of its words
+// and the warps' own dependent steps per tile fill the rest, so four warps per
+// scheduler with two row tiles are faster than two with three (6.8 ms, also
+// with the scatter of a tile behind the products of the next).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -33,11 +39,11 @@
 
 namespace dgv {
 
-constexpr int VJ_WARPS = 8;
-constexpr int VJ_NT = 3;              // row tiles of 8 per item
-constexpr int VJ_S = 8 * VJ_NT + 2;   // row stride of the per-node arrays: lanes (4 pairs x 4 rows) hit 16 banks of 8 B
-constexpr int VJ_NST = 3;             // ring stages per warp, two tiles each
-constexpr int VJ_MAXT = 128;          // tiles per block, at most: 27 nodes l1 x 4
+constexpr int VJ_WARPS = 16;
+constexpr int VJ_NT = 2;              // row tiles of 8 per item
+constexpr int VJ_S = 8 * VJ_NT + 4;   // row stride of the per-node arrays: lanes (4 pairs x 4 rows) hit 16 banks of 8 B
+constexpr int VJ_NST = 3;             // ring stages per warp, a tile each
+constexpr int VJ_MAXT = 108;          // tiles per block, at most: 27 nodes l1 x 4
 
 struct __align__(16) VjpItem {
     int block, row0, nrow, pad;
@@ -67,10 +73,10 @@ __device__ __forceinline__ void vjp_dmma(double &c0, double &c1, double a, doubl
 }
 
 #define VJP_ALIGN(x) (((x) + 15) / 16 * 16)
-// bytes of one warp's shared memory: ring, F1 | G1, F2, G2, tile list, barriers
+// bytes of one warp's shared memory: ring, F2, G2, tile list, barriers
 __host__ __device__ constexpr int vjp_warp_bytes(int P, int rowb)
 {
-    return VJP_ALIGN(VJ_NST * 16 * rowb) + 3 * VJP_ALIGN(P * VJ_S * 8) + VJ_MAXT * 4 + VJP_ALIGN(VJ_NST * 8);
+    return VJP_ALIGN(VJ_NST * 8 * rowb) + 2 * VJP_ALIGN(P * VJ_S * 8) + VJ_MAXT * 4 + VJP_ALIGN(VJ_NST * 8);
 }
 
 template <int P>
@@ -83,8 +89,8 @@ __global__ void __launch_bounds__(32 * VJ_WARPS, 1) k_vjp_mma(const __grid_const
     const int q = lane & 3, r8 = lane >> 2;
     unsigned char *smem = smem_all + warp * vjp_warp_bytes(P, a.rowb);
     unsigned char *ring = smem;
-    double *F1 = reinterpret_cast<double *>(smem + VJP_ALIGN(VJ_NST * 16 * a.rowb));  // f(c1+D, l); then g of it
-    double *F2 = F1 + VJP_ALIGN(P * VJ_S * 8) / 8, *G2 = F2 + VJP_ALIGN(P * VJ_S * 8) / 8;
+    double *F2 = reinterpret_cast<double *>(smem + VJP_ALIGN(VJ_NST * 8 * a.rowb));  // f(c2+D, l2) per row
+    double *G2 = F2 + VJP_ALIGN(P * VJ_S * 8) / 8;                                     // sums for it
     unsigned *tl = reinterpret_cast<unsigned *>(G2 + VJP_ALIGN(P * VJ_S * 8) / 8);
     uint64_t *full = reinterpret_cast<uint64_t *>(tl + VJ_MAXT);
     if (lane == 0) {
@@ -106,21 +112,18 @@ __global__ void __launch_bounds__(32 * VJ_WARPS, 1) k_vjp_mma(const __grid_const
         const int o1c = bi.c1 - a.ccell, o2c = bi.c2 - a.ccell;
         for (int t = lane; t < nt; t += 32) tl[t] = __ldg(a.tiles + t0 + t);
         __syncwarp();
-        const int nst = (nt + 1) / 2;
-        int sent = 0;
-        auto send = [&]() {  // the next two tiles' rows (consecutive) into the ring
-            if (sent >= nst) return;
+        int sent = 0, sslot = slot;
+        auto send = [&]() {  // the next tile's rows into the ring
+            if (sent >= nt) return;
             if (lane == 0) {
-                const unsigned x = tl[2 * sent];
-                int n = (int)(x >> 10 & 15u);
-                if (2 * sent + 1 < nt) n += (int)(tl[2 * sent + 1] >> 10 & 15u);
-                int at = slot + sent;  // slot: ring slot of the item's first stage
-                at %= VJ_NST;
-                mbar_arrive_expect_tx(&full[at], (uint32_t)(n * a.rowb));
-                bulk_g2s(ring + at * 16 * a.rowb, a.rows + (size_t)(bi.start + (x & 1023u)) * a.rowb, (uint32_t)(n * a.rowb),
-                         &full[at]);
+                const unsigned x = tl[sent];
+                const int n = (int)(x >> 10 & 15u);
+                mbar_arrive_expect_tx(&full[sslot], (uint32_t)(n * a.rowb));
+                bulk_g2s(ring + sslot * 8 * a.rowb, a.rows + (size_t)(bi.start + (x & 1023u)) * a.rowb,
+                         (uint32_t)(n * a.rowb), &full[sslot]);
             }
             sent++;
+            sslot = sslot + 1 == VJ_NST ? 0 : sslot + 1;
         };
         for (int s = 0; s < VJ_NST; s++) send();
         // rows: lane l has the cell of row l
@@ -131,58 +134,53 @@ __global__ void __launch_bounds__(32 * VJ_WARPS, 1) k_vjp_mma(const __grid_const
             D = ((bi.lo[0] + y / lv) * a.Mv + bi.lo[1] + y % lv) * a.Mw + bi.lo[2] + w;
         }
         const double *f = a.f + v * a.N, *cv = a.c + v * a.N;
-        // f of both cells of every row, node-major; rows past the last are zero
+        // f of cell c2 + D of every row, node-major; rows past the last are zero
 #pragma unroll 4
         for (int r = 0; r < 8 * VJ_NT; r++) {
             const int Dr = __shfl_sync(ALL, D, r);
             if (lane < P) {
-                const bool live = r < im.nrow;
-                F1[lane * VJ_S + r] = live ? __ldg(f + (size_t)(Dr + o1c) * P + lane) : 0.0;
-                F2[lane * VJ_S + r] = live ? __ldg(f + (size_t)(Dr + o2c) * P + lane) : 0.0;
+                F2[lane * VJ_S + r] = r < im.nrow ? __ldg(f + (size_t)(Dr + o2c) * P + lane) : 0.0;
                 G2[lane * VJ_S + r] = 0.0;
             }
         }
         // A fragments: c of row 8 i + r8, node q + 4 t
         double cf[VJ_NT][KT];
+        long long n1[VJ_NT];  // first node of cell c1 + D of this lane's rows; -1: no row
 #pragma unroll
         for (int i = 0; i < VJ_NT; i++) {
             const int Dr = __shfl_sync(ALL, D, 8 * i + r8);
+            n1[i] = 8 * i + r8 < im.nrow ? (long long)(Dr + o1c) * P : -1;
 #pragma unroll
             for (int t = 0; t < KT; t++)
                 cf[i][t] = 8 * i + r8 < im.nrow && q + 4 * t < P ? __ldg(cv + (size_t)Dr * P + q + 4 * t) : 0.0;
         }
         __syncwarp();
+        double *g = a.g + v * a.N;
         double y1[VJ_NT], f1[VJ_NT];
         bool fresh = true;  // the next tile begins an l1
-        unsigned m1 = 0;    // nodes l1 met
-        for (int t = 0; t < nt; t++) {
-            int st = slot + (t >> 1), ph = phase;
-            if (st >= VJ_NST) { ph ^= (st / VJ_NST) & 1; st %= VJ_NST; }
-            if ((t & 1) == 0) {
-                const bool got = mbar_wait(&full[st], (uint32_t)ph, a.err, a.wait_ns);
-                if (!__all_sync(ALL, got)) { ok = false; break; }
-            }
+        int t = 0;
+        for (; t < nt; t++) {
+            const bool got = mbar_wait(&full[slot], (uint32_t)phase, a.err, a.wait_ns);
+            if (!__all_sync(ALL, got)) { ok = false; break; }
             const unsigned x = tl[t];
             const int n = (int)(x >> 10 & 15u), l1 = (int)(x >> 14 & 31u);
-            const unsigned char *rows = ring + (st * 16 + ((t & 1) ? (int)(tl[t - 1] >> 10 & 15u) : 0)) * a.rowb;
-            // V fragments: pair r8, node q + 4 t (past P the row's last: times a zero of cf)
+            const unsigned char *rows = ring + slot * 8 * a.rowb;
+            if (fresh) {
+#pragma unroll
+                for (int i = 0; i < VJ_NT; i++) {
+                    f1[i] = n1[i] >= 0 ? __ldg(f + n1[i] + l1) : 0.0;
+                    y1[i] = 0.0;
+                }
+            }
+            // V fragments: pair r8, node q + 4 k (past P the row's last: times a zero of cf)
             const double *vr = reinterpret_cast<const double *>(rows + min(r8, n - 1) * a.rowb) + 1;
             double b[KT];
 #pragma unroll
             for (int k = 0; k < KT; k++) b[k] = vr[4 * k + 4 > P ? min(q + 4 * k, P - 1) : q + 4 * k];
             // nodes l2 of the pairs 2 q, 2 q + 1 (this lane's columns)
             const bool p0 = 2 * q < n, p1 = 2 * q + 1 < n;
-            int l20 = 0, l21 = 0;
-            if (p0) l20 = node(reinterpret_cast<const int *>(rows + 2 * q * a.rowb)[1] - o2c) * VJ_S + r8;
-            if (p1) l21 = node(reinterpret_cast<const int *>(rows + (2 * q + 1) * a.rowb)[1] - o2c) * VJ_S + r8;
-            if (fresh) {
-#pragma unroll
-                for (int i = 0; i < VJ_NT; i++) {
-                    f1[i] = F1[l1 * VJ_S + 8 * i + r8];
-                    y1[i] = 0.0;
-                }
-                m1 |= 1u << l1;
-            }
+            const int l20 = node(reinterpret_cast<const int *>(rows + min(2 * q, n - 1) * a.rowb)[1] - o2c) * VJ_S + r8;
+            const int l21 = node(reinterpret_cast<const int *>(rows + min(2 * q + 1, n - 1) * a.rowb)[1] - o2c) * VJ_S + r8;
             double acc[VJ_NT][2];
 #pragma unroll
             for (int i = 0; i < VJ_NT; i++) acc[i][0] = acc[i][1] = 0.0;
@@ -205,32 +203,35 @@ __global__ void __launch_bounds__(32 * VJ_WARPS, 1) k_vjp_mma(const __grid_const
                 }
             }
             fresh = (x >> 19 & 1u) != 0;
-            if (fresh) {  // the l1 ends: its sums replace its f (every lane holds what it needs of that)
+            if (fresh) {  // the l1 ends
 #pragma unroll
                 for (int i = 0; i < VJ_NT; i++) {
                     y1[i] += __shfl_xor_sync(ALL, y1[i], 1);
                     y1[i] += __shfl_xor_sync(ALL, y1[i], 2);
-                    if (q == 0) F1[l1 * VJ_S + 8 * i + r8] = y1[i];
+                    if (q == 0 && n1[i] >= 0) atomicAdd(g + n1[i] + l1, y1[i]);
                 }
             }
-            __syncwarp();  // G2 of this tile before the next tile's; the rows are read
-            if ((t & 1) || t + 1 == nt) send();
+            if (++slot == VJ_NST) {
+                slot = 0;
+                phase ^= 1;
+            }
+            __syncwarp();  // G2 of this tile before the next one's; the rows are read
+            send();
         }
-        if (!ok) {  // let the copies already issued land
-            for (int s = 0; s < min(sent, VJ_NST); s++) {
-                const int k = sent - 1 - s, at = (slot + k) % VJ_NST;
-                mbar_wait(&full[at], (uint32_t)(phase ^ (((slot + k) / VJ_NST) & 1)), a.err, a.wait_ns);
+        if (!ok) {  // let the copies still in flight land: those of the tiles t .. sent - 1
+            for (; t < sent; t++) {
+                mbar_wait(&full[slot], (uint32_t)phase, a.err, a.wait_ns);
+                if (++slot == VJ_NST) {
+                    slot = 0;
+                    phase ^= 1;
+                }
             }
             break;
         }
-        phase ^= ((slot + nst) / VJ_NST) & 1;
-        slot = (slot + nst) % VJ_NST;
         if (lane == 0) id = atomicAdd(a.next, 1ULL);
-        double *g = a.g + v * a.N;
         for (int r = 0; r < im.nrow; r++) {
             const int Dr = __shfl_sync(ALL, D, r);
             if (lane < P) {
-                if (m1 >> lane & 1u) atomicAdd(g + (size_t)(Dr + o1c) * P + lane, F1[lane * VJ_S + r]);
                 const double y = G2[lane * VJ_S + r];
                 if (y != 0.0) atomicAdd(g + (size_t)(Dr + o2c) * P + lane, y);
             }
