@@ -440,11 +440,14 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_collide_mma(const __grid_cons
 // which bounds a kernel with one row and all P columns per lane (32 words for
 // 27 multiply-adds).  A product is formed by one of the four lanes that need
 // it and handed on by shuffles.
-// Measured (B200): a stage of 64 rows takes 724 SM cycles, 216 of them
-// multiply-adds; shared memory's and the shuffles' ~21 words per pair and
-// their latency bound it (two rows and all columns per lane: 655, but rows in
-// steps of 32; 12 or 16 warps of 32 rows: 405 per 32 rows).  Per Q at 21^3 with
-// projection, one cell per lane -> this kernel: 18.3 -> 3.8 ms.
+// Rows are taken in pairs by packed FP32x2 operations (multiply-adds and the
+// two-sum), half the instructions of scalar ones for the same roundings.
+// Measured (B200): a stage of 64 rows takes 630 SM cycles (724 with scalar
+// operations), 216 of them multiply-adds at the scalar rate; shared memory's
+// and the shuffles' ~21 words per pair and their latency bound it (scalar: two
+// rows and all columns per lane 655, but rows in steps of 32; 12 or 16 warps of
+// 32 rows 405 per 32 rows).  Per Q at 21^3 with projection, one cell per lane ->
+// this kernel: 18.3 -> 3.3 ms.
 constexpr int FC_WARPS = 8, FC_THREADS = 32 * FC_WARPS;
 constexpr int FC_TILE = 16, FC_MT = 4;  // rows per tile (A = 2 per tile); tiles per unit
 
@@ -466,19 +469,21 @@ struct F32F {
 };
 
 // the n pairs of one group added into (sum, correction); d1, d2: places of the
-// cells whose products this lane forms (rows rg + 8 pg and rg + 8 pg + 32)
+// cells whose products this lane forms (rows rg + 8 pg and rg + 8 pg + 32).
+// Rows rg + 16 j and rg + 16 j + 8 share packed operations: each half rounds
+// like the scalar one.
 template <int P, int A, bool GF>
-__device__ __forceinline__ void f32_stage(const unsigned char *st, int n, int d1, int d2, float (*sm)[(P + 3) / 4],
-                                          float (*cr)[(P + 3) / 4], const F32F<GF> &F)
+__device__ __forceinline__ void f32_stage(const unsigned char *st, int n, int d1, int d2, float2 (*sm)[(P + 3) / 4],
+                                          float2 (*cr)[(P + 3) / 4], const F32F<GF> &F)
 {
     constexpr int RB = ((2 + P) + 3) / 4 * 16;  // bytes of a row: offsets, values, zeros
     constexpr int PB = (P + 3) / 4;
     const int pg = threadIdx.x & 3;
-    float part[A][PB];
+    float2 part[A / 2][PB];
 #pragma unroll
-    for (int j = 0; j < A; j++)
+    for (int j = 0; j < A / 2; j++)
 #pragma unroll
-        for (int i = 0; i < PB; i++) part[j][i] = 0.f;
+        for (int i = 0; i < PB; i++) part[j][i] = make_float2(0.f, 0.f);
 #pragma unroll 4
     for (int k = 0; k < n; k++) {
         const int2 o = *reinterpret_cast<const int2 *>(st + k * RB);
@@ -490,18 +495,21 @@ __device__ __forceinline__ void f32_stage(const unsigned char *st, int n, int d1
 #pragma unroll
         for (int i = 0; i < PB; i++) v[i] = row[i];
 #pragma unroll
-        for (int j = 0; j < A; j++) {
-            const float x = __shfl_sync(0xffffffffu, j < 4 ? x1 : x2, j & 3, 4);
+        for (int j = 0; j < A; j += 2) {
+            const float xl = j < 4 ? x1 : x2;
+            const float2 x = make_float2(__shfl_sync(0xffffffffu, xl, j & 3, 4), __shfl_sync(0xffffffffu, xl, j + 1 & 3, 4));
 #pragma unroll
-            for (int i = 0; i < PB; i++) part[j][i] = fmaf(v[i], x, part[j][i]);
+            for (int i = 0; i < PB; i++) part[j / 2][i] = __ffma2_rn(make_float2(v[i], v[i]), x, part[j / 2][i]);
         }
     }
+    const float2 m1 = make_float2(-1.f, -1.f);
 #pragma unroll
-    for (int j = 0; j < A; j++)
+    for (int j = 0; j < A / 2; j++)
 #pragma unroll
         for (int i = 0; i < PB; i++) {  // two-sum: sum + correction carries the group sum exactly
-            const float x = part[j][i], s = sm[j][i], t = s + x, bp = t - s;
-            cr[j][i] += (s - (t - bp)) + (x - bp);
+            const float2 x = part[j][i], s = sm[j][i], t = __fadd2_rn(s, x), bp = __ffma2_rn(s, m1, t);
+            const float2 e = __fadd2_rn(__ffma2_rn(__ffma2_rn(bp, m1, t), m1, s), __ffma2_rn(bp, m1, x));
+            cr[j][i] = __fadd2_rn(cr[j][i], e);
             sm[j][i] = t;
         }
 }
@@ -544,11 +552,11 @@ __global__ void __launch_bounds__(FC_THREADS, 1) k_collide_f32(const __grid_cons
             const int r = 32 * warp + lane;
             rowcell[r] = mma_cell(un, un.row0 + min(r, un.nrow - 1), a.Mv, a.Mw) - a.cell0;
         }
-        float sm[2 * FC_MT][PB], cr[2 * FC_MT][PB];
+        float2 sm[FC_MT][PB], cr[FC_MT][PB];  // rows rg + 16 j, rg + 16 j + 8
 #pragma unroll
-        for (int j = 0; j < 2 * FC_MT; j++)
+        for (int j = 0; j < FC_MT; j++)
 #pragma unroll
-            for (int i = 0; i < PB; i++) sm[j][i] = cr[j][i] = 0.f;
+            for (int i = 0; i < PB; i++) sm[j][i] = cr[j][i] = make_float2(0.f, 0.f);
         const int nmine = (sb - sa - warp + FC_WARPS - 1) / FC_WARPS;
 #define DGV_F32_CASE(NT)                                                    \
     case NT:                                                                \
@@ -575,7 +583,8 @@ __global__ void __launch_bounds__(FC_THREADS, 1) k_collide_f32(const __grid_cons
             const bool mine = row < 8 && 8 * j + row < un.nrow;
 #pragma unroll
             for (int i = 0; i < PB; i++)
-                red[(size_t)(warp * 8 + rg) * CW + PB * pg + i] = (double)sm[j][i] + (double)cr[j][i];
+                red[(size_t)(warp * 8 + rg) * CW + PB * pg + i] =
+                    j & 1 ? (double)sm[j / 2][i].y + (double)cr[j / 2][i].y : (double)sm[j / 2][i].x + (double)cr[j / 2][i].x;
             __syncthreads();
             if (mine) {
                 double *dst = part + (size_t)rowcell[8 * j + row] * P + p;
