@@ -163,6 +163,14 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity, i
     return __all_sync(0xffffffffu, ok);
 }
 
+// true in one lane of the converged warp, the same one each time
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.b32 %0, 1, 0, q;\n\t}" : "=r"(p));
+    return p != 0;
+}
+
 // split x into fp16 hi + lo (two values at a time)
 __device__ __forceinline__ void split2(float x0, float x1, uint32_t &hi, uint32_t &lo)
 {
@@ -791,7 +799,7 @@ static int tc_lists(Ctx *c, int NDG, TcLists *out)
 // VDF tiles, so each block's W crosses from L2 once for 256 rows.
 // Warp roles (320 threads, one CTA per SM):
 //   warp 0     producer: TMA bulk copies of f (both tiles) and W groups
-//   warp 1     allocates all 512 tensor-memory columns; lane 0 issues MMAs
+//   warp 1     allocates all 512 tensor-memory columns; one elected lane issues MMAs
 //   warps 2-9  epilogue: warp w serves VDF tile (w-2)/4, tensor-memory lanes
 //              32*(w%4) .. +31 (one row per thread)
 // Tensor memory: two accumulators of 256 columns, used alternately by the
@@ -1294,7 +1302,13 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_collide_tc2(const __grid_cons
         __syncwarp();
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
+        // The whole warp walks the work and waits; one elected lane issues.  In
+        // code that only lane 0 runs every operand of an MMA is a per-thread
+        // value; with the warp converged they are uniform, and the issuer keeps
+        // up with the tensor pipe beside the epilogue warps of its scheduler
+        // (B200, 21^3 x 37: 32.1 -> 29.2 ms, 14^3 x 150, 8 nodes: 22.4 -> 20.9,
+        // 27^3 x 256: 543 -> 538, adjoint 21^3 x 150: 150.8 -> 147.9).
+        {
             // FP32 accumulator, fp16 A and B, both K-major, M = 128, N = 256;
             // an item's last group holds ncol - 256 (ngb-1) columns: its MMAs
             // use N rounded up to 16
@@ -1305,16 +1319,17 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_collide_tc2(const __grid_cons
                 int u = k == 0 ? (int)blockIdx.x : total;
                 if (L.counter) {
                     const int slot = k & 1;
-                    if (!mbar_wait(&uq_full[slot], (k >> 1) & 1, err0, L.wait_ns)) { ok = false; break; }
+                    if (!mbar_wait_warp(&uq_full[slot], (k >> 1) & 1, err0, L.wait_ns)) { ok = false; break; }
                     u = uq[slot];
-                    mbar_arrive(&uq_empty[slot]);
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&uq_empty[slot]);
                 }
                 if (u >= total) break;
                 const T2Unit un = t2_unit<MG>(L, u);
                 int *const err = L.g[MG ? un.gi : 0].err;
                 for (int it = un.i0; it < un.i1 && ok; it++) {
                     const int s = q & 1;
-                    if (!mbar_wait(&s_full[s], (q >> 1) & 1, err, L.wait_ns)) { ok = false; break; }
+                    if (!mbar_wait_warp(&s_full[s], (q >> 1) & 1, err, L.wait_ns)) { ok = false; break; }
                     const int ncol = *reinterpret_cast<const int *>(slots + (size_t)(2 * s) * region + 2 * T2_ATILE +
                                                                      NDG * P * VB * 4);
                     const int ngb = (ncol + T2_N - 1) / T2_N;
@@ -1323,37 +1338,43 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_collide_tc2(const __grid_cons
                         (1u << 4) | ((uint32_t)(nlast >> 3) << 17) | ((uint32_t)(TC_ROWS >> 4) << 24);
                     for (int g = 0; g < ngb && ok; g++, gw++) {
                         const int st = gw % T2_NSTW;
-                        if (!mbar_wait(&w_full[st], (gw / T2_NSTW) & 1, err, L.wait_ns)) { ok = false; break; }
+                        if (!mbar_wait_warp(&w_full[st], (gw / T2_NSTW) & 1, err, L.wait_ns)) { ok = false; break; }
                         const uint64_t dWh = umma_desc(smem_u32(wring + st * T2_GREC), 128, 512);
                         const uint64_t dWl = umma_desc(smem_u32(wring + st * T2_GREC + T2_TILE), 128, 512);
                         const uint32_t id = g == ngb - 1 ? idesc_last : idesc;
                         for (int j = 0; j < un.nb2; j++, J++) {
                             const int cs = J & 1;
-                            if (!mbar_wait(&c_empty[cs], ((J >> 1) & 1) ^ 1, err, L.wait_ns)) { ok = false; break; }
+                            if (!mbar_wait_warp(&c_empty[cs], ((J >> 1) & 1) ^ 1, err, L.wait_ns)) { ok = false; break; }
                             tc_fence_after();
                             unsigned char *reg = slots + (size_t)(2 * s + j) * region;
                             const uint64_t dAh = umma_desc(smem_u32(reg), 128, 512);
                             const uint64_t dAl = umma_desc(smem_u32(reg + T2_ATILE), 128, 512);
                             const uint32_t dacc = tmem + (uint32_t)(cs * T2_N);
+                            if (elect_one()) {
 #pragma unroll
-                            for (int t = 0; t < T2_K / 16; t++) {  // K = 16 per instruction: 256 B along K
-                                umma_f16(dacc, dAh + 16 * t, dWh + 16 * t, id, t ? 1u : 0u);
-                                umma_f16(dacc, dAh + 16 * t, dWl + 16 * t, id, 1u);
-                                umma_f16(dacc, dAl + 16 * t, dWh + 16 * t, id, 1u);
+                                for (int t = 0; t < T2_K / 16; t++) {  // K = 16 per instruction: 256 B along K
+                                    umma_f16(dacc, dAh + 16 * t, dWh + 16 * t, id, t ? 1u : 0u);
+                                    umma_f16(dacc, dAh + 16 * t, dWl + 16 * t, id, 1u);
+                                    umma_f16(dacc, dAl + 16 * t, dWh + 16 * t, id, 1u);
+                                }
+                                umma_commit(&c_full[cs]);
                             }
-                            umma_commit(&c_full[cs]);
+                            __syncwarp();
                         }
                         if (!ok) break;
-                        umma_commit(&w_empty[st]);
+                        if (elect_one()) umma_commit(&w_empty[st]);
+                        __syncwarp();
                     }
                     if (!ok) break;
-                    umma_commit(&s_empty[s]);
+                    if (elect_one()) umma_commit(&s_empty[s]);
+                    __syncwarp();
                     q++;
                 }
             }
             // every MMA issued so far completes before tensor memory is freed
-            umma_commit(drain);
-            mbar_wait(drain, 0, err0, L.wait_ns);
+            if (elect_one()) umma_commit(drain);
+            __syncwarp();
+            mbar_wait_warp(drain, 0, err0, L.wait_ns);
         }
         __syncwarp();
     } else if ((warp - 2) / 4 < nbw) {
