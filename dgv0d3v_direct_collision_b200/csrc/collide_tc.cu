@@ -156,10 +156,11 @@ __device__ __forceinline__ float2 fmul2(float2 a, float2 b)
 
 // bounded wait whose outcome is the same for every lane of the warp (the
 // warp-collective tensor-memory instructions that follow need a converged warp)
+template <uint32_t HOLD = 0>
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity, int *err,
                                                unsigned long long limit_ns = WAIT_LIMIT_NS)
 {
-    const bool ok = mbar_wait(bar, parity, err, limit_ns);
+    const bool ok = mbar_wait<HOLD>(bar, parity, err, limit_ns);
     return __all_sync(0xffffffffu, ok);
 }
 
@@ -807,12 +808,25 @@ static int tc_lists(Ctx *c, int NDG, TcLists *out)
 // at N = 128 whether A comes from shared or tensor memory, and about the same
 // at N = 256, so the wide groups halve the MMA time of a block.  Every wait is
 // bounded, as in the chunk form.
-constexpr int T2_N = 256;                     // columns (l1, p) per group
-constexpr int T2_K = 32;                      // nodes l2 per block, zero-padded
-constexpr int T2_TILE = T2_N * T2_K * 2;      // one fp16 tile (16 KiB)
-constexpr int T2_GREC = 2 * T2_TILE;          // hi and lo tiles of one group
-constexpr int T2_NSTW = 3;                    // W ring stages
-constexpr int T2_ATILE = TC_ROWS * T2_K * 2;  // 128 rows x 32 fp16 (8 KiB)
+//
+// Eight nodes per cell: a block is one group of 64 columns and 8 nodes l2, so
+// its tiles are 64 x 16 (K = 16, one MMA per split product instead of two) and
+// its record 4 KB; in the 256 x 32 tiles of 27 nodes 15/16 of the 32 KB copied
+// per block were zeros.  An item is then a few hundred cycles of work for each
+// role, less than the latency of its copies, so what shared and tensor memory
+// the small tiles leave goes to four item slots, eight W stages and eight
+// accumulators of 64 columns, and the producer loads an item one ahead.  With
+// long holds in the waits (HOLD below) 14^3 x 150 takes 19.0 ms, 20.9 in the
+// tiles of 27 nodes: an item's chain of waits bounds it, ~2,000 cycles.
+__host__ __device__ constexpr int t2_n(int P) { return P == 8 ? 64 : 256; }        // columns (l1, p) per group
+__host__ __device__ constexpr int t2_k(int P) { return P == 8 ? 16 : 32; }         // nodes l2 per block, zero-padded
+__host__ __device__ constexpr int t2_tile(int P) { return t2_n(P) * t2_k(P) * 2; }  // one fp16 tile (16 KiB; 2 KiB)
+__host__ __device__ constexpr int t2_grec(int P) { return 2 * t2_tile(P); }        // hi and lo tiles of one group
+__host__ __device__ constexpr int t2_atile(int P) { return TC_ROWS * t2_k(P) * 2; }  // 128 rows x K fp16 (8 KiB; 4 KiB)
+__host__ __device__ constexpr int t2_nstw(int P) { return P == 8 ? 8 : 3; }        // W ring stages
+__host__ __device__ constexpr int t2_nslot(int P) { return P == 8 ? 4 : 2; }       // item slots
+__host__ __device__ constexpr int t2_nacc(int P) { return 512 / t2_n(P); }         // accumulators in tensor memory
+constexpr int T2_SETREC = 32 * 1024;  // bytes that a column group counts in the size of a block set, whatever P
 constexpr int T2_EPI_WARPS = 8;
 // slot header, after the side tile of the slot's first VDF tile: the item's
 // column count, for each rank jj of its mask the offset (floats) l*VB of the
@@ -821,22 +835,22 @@ constexpr int T2_EPI_WARPS = 8;
 constexpr int T2_HDR = 128;
 constexpr int T2_THREADS = 32 * (2 + T2_EPI_WARPS);
 
-__host__ __device__ constexpr int t2_groups(int P) { return (P * P + T2_N - 1) / T2_N; }
+__host__ __device__ constexpr int t2_groups(int P) { return (P * P + t2_n(P) - 1) / t2_n(P); }
 
 // column groups of a collision-operator item: its block's mask of nodes l1
 // is in the low 27 bits of nch
 template <int P>
 __device__ __forceinline__ int t2_item_groups(int nch)
 {
-    return (__popc((unsigned)nch & 0x7ffffffu) * P + T2_N - 1) / T2_N;
+    return (__popc((unsigned)nch & 0x7ffffffu) * P + t2_n(P) - 1) / t2_n(P);
 }
 
-// byte offset of element (row, k) of a K-major tile without swizzle, K = 32:
-// core matrices of 8 rows x 16 bytes, four along K (128 B apart), row groups
-// of 8 512 B apart
-__host__ __device__ __forceinline__ int t2_off(int row, int k)
+// byte offset of element (row, k) of a K-major tile without swizzle: core
+// matrices of 8 rows x 16 bytes, K / 8 along K (128 B apart), row groups of 8
+// 16 K bytes apart
+__host__ __device__ __forceinline__ int t2_off(int row, int k, int K)
 {
-    return ((row >> 3) * 4 + (k >> 3)) * 128 + (row & 7) * 16 + (k & 7) * 2;
+    return ((row >> 3) * (K >> 3) + (k >> 3)) * 128 + (row & 7) * 16 + (k & 7) * 2;
 }
 
 // per block the masks of the nodes l1 (mask[b]) and l2 (mask[nblocks + b])
@@ -866,21 +880,22 @@ __global__ void k_tc2_mask(const BlockInfo *blk, const double *rows64, int RD64,
 }
 
 // one record per block: groups of {W hi tile, W lo tile}, group g holding
-// columns n in [256 g, 256 g + 256) as tile rows, compacted to the nodes of
+// columns n in [N g, N g + N) as tile rows (N = t2_n), compacted to the nodes of
 // one of the block's masks: arrangement 0 (the collision operator and the
 // adjoint's pass to the c1 side) n = rank(l1)*P + p, K = l2, mask of the
 // nodes l1; arrangement 1 (the adjoint's pass to the c2 side) n = rank(l2)*P +
 // p, K = l1, mask of the nodes l2.  The block's record holds goff[b+1] -
-// goff[b] = ceil(popc(mask) P / 256) groups from group goff[b] on.
+// goff[b] = ceil(popc(mask) P / N) groups from group goff[b] on.
 __global__ void k_tc2_build(const BlockInfo *blk, const double *rows64, int RD64, int P, int Nc, int ccell,
                             float vscale, unsigned char *W, int arr, const unsigned *mask, const long long *goff)
 {
     const BlockInfo bi = blk[blockIdx.x];
     const int NG = (int)(goff[blockIdx.x + 1] - goff[blockIdx.x]);
+    const int N = t2_n(P), grec = t2_grec(P);
     const unsigned msk = mask[blockIdx.x];
-    unsigned char *rec = W + (size_t)goff[blockIdx.x] * T2_GREC;
+    unsigned char *rec = W + (size_t)goff[blockIdx.x] * grec;
     uint4 *r4 = reinterpret_cast<uint4 *>(rec);
-    for (int t = threadIdx.x; t < NG * T2_GREC / 16; t += blockDim.x) r4[t] = make_uint4(0u, 0u, 0u, 0u);
+    for (int t = threadIdx.x; t < NG * grec / 16; t += blockDim.x) r4[t] = make_uint4(0u, 0u, 0u, 0u);
     __syncthreads();
     for (int t = threadIdx.x; t < bi.count * P; t += blockDim.x) {
         const int k = t / P, p = t - k * P;
@@ -889,18 +904,18 @@ __global__ void k_tc2_build(const BlockInfo *blk, const double *rows64, int RD64
         const int o1 = (int)(unsigned)(o & 0xffffffffLL), o2 = (int)(o >> 32);
         const int l1 = (o1 - (bi.c1 - ccell)) / Nc, l2 = (o2 - (bi.c2 - ccell)) / Nc;
         const int lc = arr == 0 ? l1 : l2, lk = arr == 0 ? l2 : l1;
-        const int n = __popc(msk & ((1u << lc) - 1u)) * P + p, g = n / T2_N;
+        const int n = __popc(msk & ((1u << lc) - 1u)) * P + p, g = n / N;
         const float x = (float)(row[1 + p] * (double)vscale);
         const __half h = __float2half_rn(x);
         const __half l = __float2half_rn(x - __half2float(h));
-        unsigned char *dst = rec + (size_t)g * T2_GREC + t2_off(n - g * T2_N, lk);
+        unsigned char *dst = rec + (size_t)g * grec + t2_off(n - g * N, lk, t2_k(P));
         *reinterpret_cast<__half *>(dst) = h;
-        *reinterpret_cast<__half *>(dst + T2_TILE) = l;
+        *reinterpret_cast<__half *>(dst + t2_tile(P)) = l;
     }
 }
 
-// F16[((bt*2 + h)*Nc + cell) * VB*64 + t2_off(v, l)]: per VDF tile and cell a
-// tile of VB rows (VDFs) x 32 nodes, h = 0 hi / 1 lo parts of the scaled FP32
+// F16[((bt*2 + h)*Nc + cell) * VB*2*K + t2_off(v, l, K)]: per VDF tile and cell
+// a tile of VB rows (VDFs) x K = t2_k(P) nodes, h = 0 hi / 1 lo parts of the scaled FP32
 // copy F[((bt*Nc + cell)*P + l)*VB + v]; nodes l >= P are zero
 constexpr int T2_MAXG = 4;  // grids of one launch (mixed-grid batches)
 
@@ -952,10 +967,10 @@ __global__ void k_tc2_prep(const __grid_constant__ Tc2PrepLaunch A)
     }
     const double sc = ldexp(1.0, e);
     if (threadIdx.x == 0) G.inv_scale[v] = ldexp(1.0, -G.pw * e) * G.vinv;
-    const int bt = v / G.VB, lb = v % G.VB, P = G.P;
-    const size_t tile = (size_t)G.VB * T2_K * 2;
-    for (long long i = threadIdx.x; i < (long long)G.Nc * T2_K; i += blockDim.x) {
-        const int cell = (int)(i / T2_K), l = (int)(i % T2_K);
+    const int bt = v / G.VB, lb = v % G.VB, P = G.P, K = t2_k(P);
+    const size_t tile = (size_t)G.VB * K * 2;
+    for (long long i = threadIdx.x; i < (long long)G.Nc * K; i += blockDim.x) {
+        const int cell = (int)(i / K), l = (int)(i % K);
         float x = 0.f;
         if (l < P) {
             x = v < G.nvdf ? (float)(G.f[(size_t)v * G.N + (size_t)cell * P + l] * sc) : 0.f;
@@ -963,7 +978,7 @@ __global__ void k_tc2_prep(const __grid_constant__ Tc2PrepLaunch A)
         }
         const __half h = __float2half_rn(x);
         const __half lo = __float2half_rn(x - __half2float(h));
-        unsigned char *base = G.F16 + ((size_t)(2 * bt) * G.Nc + cell) * tile + t2_off(lb, l);
+        unsigned char *base = G.F16 + ((size_t)(2 * bt) * G.Nc + cell) * tile + t2_off(lb, l, K);
         *reinterpret_cast<__half *>(base) = h;
         *reinterpret_cast<__half *>(base + (size_t)G.Nc * tile) = lo;
     }
@@ -1002,7 +1017,7 @@ __global__ void k_tc2_final(const __grid_constant__ Tc2FinalLaunch A)
 
 struct Tc2Args {
     const float *F;            // [nbt][Nc][P][VB] FP32 side factor: scaled f (forward) or c = 2v/w (adjoint)
-    const unsigned char *F16;  // [nbt][hi, lo][Nc][VB x 32 tile]
+    const unsigned char *F16;  // [nbt][hi, lo][Nc][VB x K tile]
     const unsigned char *W;    // block records
     const unsigned char *W2;   // adjoint: the records of its pass to the c2 side (items with 1 << 30)
     const TcItem *items;       // work lists (chunk0 = first record group, | 1 << 30 for W2)
@@ -1140,16 +1155,22 @@ template <int VB, int P, int MODE, bool MG>
 __global__ void __launch_bounds__(T2_THREADS, 1) k_collide_tc2(const __grid_constant__ Tc2Launch L)
 {
     constexpr int NDG = TC_ROWS / VB;
-    constexpr int NG = t2_groups(P);
+    constexpr int NG = t2_groups(P), T2_N = t2_n(P), T2_K = t2_k(P), T2_TILE = t2_tile(P), T2_GREC = t2_grec(P);
+    constexpr int T2_ATILE = t2_atile(P), T2_NSTW = t2_nstw(P), NSLOT = t2_nslot(P), NACC = t2_nacc(P);
+    // Long holds suit the short items of 8 nodes per cell (14^3 x 150: 20.8 ms
+    // with the default, 19.0 with 50 us) and not those of 27 (27^3 x 256: 537 ms
+    // with the default, 546 with 50 us)
+    constexpr uint32_t HOLD = P == 8 ? 50000 : 0;
+    constexpr int SBO = 16 * T2_K;  // row groups of 8 of a tile
     extern __shared__ __align__(1024) unsigned char smem[];
     const int region = L.region;
     unsigned char *wring = smem;                      // T2_NSTW x T2_GREC
-    unsigned char *slots = smem + T2_NSTW * T2_GREC;  // 2 item slots x 2 VDF tiles x region
-    uint64_t *bars = reinterpret_cast<uint64_t *>(slots + 4 * region);
+    unsigned char *slots = smem + T2_NSTW * T2_GREC;  // NSLOT item slots x 2 VDF tiles x region
+    uint64_t *bars = reinterpret_cast<uint64_t *>(slots + 2 * NSLOT * region);
     uint64_t *w_full = bars, *w_empty = bars + T2_NSTW;
-    uint64_t *s_full = w_empty + T2_NSTW, *s_empty = s_full + 2;
-    uint64_t *c_full = s_empty + 2, *c_empty = c_full + 2;
-    uint64_t *drain = c_empty + 4;
+    uint64_t *s_full = w_empty + T2_NSTW, *s_empty = s_full + NSLOT;
+    uint64_t *c_full = s_empty + NSLOT, *c_empty = c_full + NACC;
+    uint64_t *drain = c_empty + NACC;
     uint64_t *uq_full = drain + 1, *uq_empty = uq_full + 2;  // unit queue
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(uq_empty + 2);
     volatile int *uq = reinterpret_cast<volatile int *>(tmem_slot + 1);
@@ -1166,11 +1187,11 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_collide_tc2(const __grid_cons
             mbar_init(&w_full[s], 1);
             mbar_init(&w_empty[s], 1);
         }
-        for (int s = 0; s < 2; s++) {
+        for (int s = 0; s < NSLOT; s++) {
             mbar_init(&s_full[s], 1);
             mbar_init(&s_empty[s], 1 + 4 * nbw);  // the MMA commit + the epilogue warps of the CTA's tiles
         }
-        for (int s = 0; s < 2; s++) {
+        for (int s = 0; s < NACC; s++) {
             mbar_init(&c_full[s], 1);
             mbar_init(&c_empty[s], 4);  // the epilogue warps of the job's tile
         }
@@ -1194,7 +1215,7 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_collide_tc2(const __grid_cons
     // grid, so rows of such cells read what the slot held before -- zeros or
     // finite values of earlier items, which the zero side factors of rows an
     // item does not serve turn into exact zeros
-    for (int t = threadIdx.x; t < region / 4; t += blockDim.x)  // 4 slots of `region` bytes, 16 B per store
+    for (int t = threadIdx.x; t < 2 * NSLOT * region / 16; t += blockDim.x)  // 16 B per store
         reinterpret_cast<uint4 *>(slots)[t] = make_uint4(0u, 0u, 0u, 0u);
     fence_async_shared();  // visible to the tensor core and ordered before the copies
     if (warp >= 2) {
@@ -1222,7 +1243,7 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_collide_tc2(const __grid_cons
                 if (L.counter) {
                     // hand the next unit to the other roles (a unit >= total ends them)
                     const int slot = k & 1;
-                    if (!mbar_wait(&uq_empty[slot], ((k >> 1) & 1) ^ 1, err0, L.wait_ns)) { ok = false; break; }
+                    if (!mbar_wait<HOLD>(&uq_empty[slot], ((k >> 1) & 1) ^ 1, err0, L.wait_ns)) { ok = false; break; }
                     u = atomicAdd(L.counter, 1);
                     uq[slot] = u;
                     mbar_arrive(&uq_full[slot]);
@@ -1231,10 +1252,12 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_collide_tc2(const __grid_cons
                 const T2Unit un = t2_unit<MG>(L, u);
                 const Tc2Args &a = L.g[MG ? un.gi : 0];
                 const int D0 = un.tile * NDG;
+                TcItem en = un.i0 < un.i1 ? a.items[un.i0] : TcItem{};
                 for (int it = un.i0; it < un.i1; it++) {
-                    const TcItem e = a.items[it];
-                    const int s = q & 1;
-                    if (!mbar_wait(&s_empty[s], ((q >> 1) & 1) ^ 1, a.err, L.wait_ns)) { ok = false; break; }
+                    const TcItem e = en;
+                    if (it + 1 < un.i1) en = a.items[it + 1];
+                    const int s = q % NSLOT;
+                    if (!mbar_wait<HOLD>(&s_empty[s], ((q / NSLOT) & 1) ^ 1, a.err, L.wait_ns)) { ok = false; break; }
                     // f of cells c1 + D - ccell (FP32) and c2 + D - ccell (fp16
                     // tiles), D in the row tile, clipped to the grid
                     const int cs1 = e.c1 + D0 - a.ccell, cs2 = e.c2 + D0 - a.ccell;
@@ -1282,7 +1305,7 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_collide_tc2(const __grid_cons
                         ((MODE == 1 && (e.chunk0 >> 30)) ? a.W2 : a.W) + (size_t)(e.chunk0 & 0x3fffffff) * T2_GREC;
                     for (int g = 0; g < ngb; g++, gw++) {
                         const int st = gw % T2_NSTW;
-                        if (!mbar_wait(&w_empty[st], ((gw / T2_NSTW) & 1) ^ 1, a.err, L.wait_ns)) {
+                        if (!mbar_wait<HOLD>(&w_empty[st], ((gw / T2_NSTW) & 1) ^ 1, a.err, L.wait_ns)) {
                             ok = false;
                             break;
                         }
@@ -1295,8 +1318,9 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_collide_tc2(const __grid_cons
             }
             if (!ok) {  // let the copies already issued land
                 for (int j = gw > T2_NSTW ? gw - T2_NSTW : 0; j < gw; j++)
-                    mbar_wait(&w_full[j % T2_NSTW], (j / T2_NSTW) & 1, err0, L.wait_ns);
-                for (int j = q > 2 ? q - 2 : 0; j < q; j++) mbar_wait(&s_full[j & 1], (j >> 1) & 1, err0, L.wait_ns);
+                    mbar_wait<HOLD>(&w_full[j % T2_NSTW], (j / T2_NSTW) & 1, err0, L.wait_ns);
+                for (int j = q > NSLOT ? q - NSLOT : 0; j < q; j++)
+                    mbar_wait<HOLD>(&s_full[j % NSLOT], (j / NSLOT) & 1, err0, L.wait_ns);
             }
         }
         __syncwarp();
@@ -1319,7 +1343,7 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_collide_tc2(const __grid_cons
                 int u = k == 0 ? (int)blockIdx.x : total;
                 if (L.counter) {
                     const int slot = k & 1;
-                    if (!mbar_wait_warp(&uq_full[slot], (k >> 1) & 1, err0, L.wait_ns)) { ok = false; break; }
+                    if (!mbar_wait_warp<HOLD>(&uq_full[slot], (k >> 1) & 1, err0, L.wait_ns)) { ok = false; break; }
                     u = uq[slot];
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&uq_empty[slot]);
@@ -1328,8 +1352,8 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_collide_tc2(const __grid_cons
                 const T2Unit un = t2_unit<MG>(L, u);
                 int *const err = L.g[MG ? un.gi : 0].err;
                 for (int it = un.i0; it < un.i1 && ok; it++) {
-                    const int s = q & 1;
-                    if (!mbar_wait_warp(&s_full[s], (q >> 1) & 1, err, L.wait_ns)) { ok = false; break; }
+                    const int s = q % NSLOT;
+                    if (!mbar_wait_warp<HOLD>(&s_full[s], (q / NSLOT) & 1, err, L.wait_ns)) { ok = false; break; }
                     const int ncol = *reinterpret_cast<const int *>(slots + (size_t)(2 * s) * region + 2 * T2_ATILE +
                                                                      NDG * P * VB * 4);
                     const int ngb = (ncol + T2_N - 1) / T2_N;
@@ -1338,17 +1362,17 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_collide_tc2(const __grid_cons
                         (1u << 4) | ((uint32_t)(nlast >> 3) << 17) | ((uint32_t)(TC_ROWS >> 4) << 24);
                     for (int g = 0; g < ngb && ok; g++, gw++) {
                         const int st = gw % T2_NSTW;
-                        if (!mbar_wait_warp(&w_full[st], (gw / T2_NSTW) & 1, err, L.wait_ns)) { ok = false; break; }
-                        const uint64_t dWh = umma_desc(smem_u32(wring + st * T2_GREC), 128, 512);
-                        const uint64_t dWl = umma_desc(smem_u32(wring + st * T2_GREC + T2_TILE), 128, 512);
+                        if (!mbar_wait_warp<HOLD>(&w_full[st], (gw / T2_NSTW) & 1, err, L.wait_ns)) { ok = false; break; }
+                        const uint64_t dWh = umma_desc(smem_u32(wring + st * T2_GREC), 128, SBO);
+                        const uint64_t dWl = umma_desc(smem_u32(wring + st * T2_GREC + T2_TILE), 128, SBO);
                         const uint32_t id = g == ngb - 1 ? idesc_last : idesc;
                         for (int j = 0; j < un.nb2; j++, J++) {
-                            const int cs = J & 1;
-                            if (!mbar_wait_warp(&c_empty[cs], ((J >> 1) & 1) ^ 1, err, L.wait_ns)) { ok = false; break; }
+                            const int cs = J % NACC;
+                            if (!mbar_wait_warp<HOLD>(&c_empty[cs], ((J / NACC) & 1) ^ 1, err, L.wait_ns)) { ok = false; break; }
                             tc_fence_after();
                             unsigned char *reg = slots + (size_t)(2 * s + j) * region;
-                            const uint64_t dAh = umma_desc(smem_u32(reg), 128, 512);
-                            const uint64_t dAl = umma_desc(smem_u32(reg + T2_ATILE), 128, 512);
+                            const uint64_t dAh = umma_desc(smem_u32(reg), 128, SBO);
+                            const uint64_t dAl = umma_desc(smem_u32(reg + T2_ATILE), 128, SBO);
                             const uint32_t dacc = tmem + (uint32_t)(cs * T2_N);
                             if (elect_one()) {
 #pragma unroll
@@ -1374,7 +1398,7 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_collide_tc2(const __grid_cons
             // every MMA issued so far completes before tensor memory is freed
             if (elect_one()) umma_commit(drain);
             __syncwarp();
-            mbar_wait_warp(drain, 0, err0, L.wait_ns);
+            mbar_wait_warp<HOLD>(drain, 0, err0, L.wait_ns);
         }
         __syncwarp();
     } else if ((warp - 2) / 4 < nbw) {
@@ -1389,7 +1413,7 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_collide_tc2(const __grid_cons
             int u = k == 0 ? (int)blockIdx.x : total;
             if (L.counter) {
                 const int slot = k & 1;
-                if (!mbar_wait_warp(&uq_full[slot], (k >> 1) & 1, err0, L.wait_ns)) { ok = false; break; }
+                if (!mbar_wait_warp<HOLD>(&uq_full[slot], (k >> 1) & 1, err0, L.wait_ns)) { ok = false; break; }
                 u = uq[slot];
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&uq_empty[slot]);
@@ -1416,8 +1440,8 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_collide_tc2(const __grid_cons
 #pragma unroll
             for (int i = 0; i < (MODE == 0 ? P2 : 1); i++) acc2[i] = make_float2(0.f, 0.f);  // MODE 0: the item's sums
             for (int it = i0; it < i1; it++) {
-                const int s = q & 1;
-                if (!mbar_wait_warp(&s_full[s], (q >> 1) & 1, err, L.wait_ns)) { ok = false; break; }
+                const int s = q % NSLOT;
+                if (!mbar_wait_warp<HOLD>(&s_full[s], (q / NSLOT) & 1, err, L.wait_ns)) { ok = false; break; }
                 const float *f1s = reinterpret_cast<const float *>(slots + (size_t)(2 * s + j) * region + 2 * T2_ATILE) +
                                    d * P * VB + v;
                 const int *hoff =
@@ -1457,8 +1481,8 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_collide_tc2(const __grid_cons
 #pragma unroll
                 for (int g = 0; g < NG; g++) {
                     if (g >= ngb) break;
-                    const int J = Jb + g * nb2 + j, cs = J & 1;
-                    if (!mbar_wait_warp(&c_full[cs], (J >> 1) & 1, err, L.wait_ns)) { ok = false; break; }
+                    const int J = Jb + g * nb2 + j, cs = J % NACC;
+                    if (!mbar_wait_warp<HOLD>(&c_full[cs], (J / NACC) & 1, err, L.wait_ns)) { ok = false; break; }
                     tc_fence_after();
 #pragma unroll
                     for (int hh = 0; hh < T2_N / LW; hh++) {
@@ -1584,8 +1608,8 @@ static int tc2_prepare(Ctx *c)
         DGV_CUDA(c, cudaStreamSynchronize(c->stream));
     }
     for (long long b = 0; b < nb; b++)
-        L.tc2_goff[b + 1] = L.tc2_goff[b] + (__builtin_popcount(L.tc2_mask[b]) * g.P + T2_N - 1) / T2_N;
-    const size_t bytes = (size_t)std::max<long long>(1, L.tc2_goff[nb]) * T2_GREC;
+        L.tc2_goff[b + 1] = L.tc2_goff[b] + (__builtin_popcount(L.tc2_mask[b]) * g.P + t2_n(g.P) - 1) / t2_n(g.P);
+    const size_t bytes = (size_t)std::max<long long>(1, L.tc2_goff[nb]) * t2_grec(g.P);
     cudaError_t e = cudaMalloc(&L.tc2_W, bytes);
     if (e != cudaSuccess || cudaMalloc(&d_goff, sizeof(long long) * (nb + 1)) != cudaSuccess) {
         cudaGetLastError();
@@ -1626,7 +1650,7 @@ static void tc2_sets(Ctx *c)
     // about tc_set_mb MB of the collision operator's (compacted) records per set
     L.tc2_sets.clear();
     L.tc2_sets.push_back(0);
-    const long long per_set = std::max<long long>(1, ((long long)c->tc_set_mb << 20) / T2_GREC);
+    const long long per_set = std::max<long long>(1, ((long long)c->tc_set_mb << 20) / T2_SETREC);
     long long acc = 0;
     for (long long b = 0; b < L.nblocks; b++) {
         acc += L.tc2_goff[b + 1] - L.tc2_goff[b];
@@ -1649,7 +1673,7 @@ static void tc2_sets_adjoint(Ctx *c)
     Layout &L = c->lay;
     if (!L.tc2_sets_adj.empty()) return;
     L.tc2_sets_adj.push_back(0);
-    const long long per_set = std::max<long long>(1, ((long long)c->tc_set_mb << 20) / T2_GREC);
+    const long long per_set = std::max<long long>(1, ((long long)c->tc_set_mb << 20) / T2_SETREC);
     long long acc = 0;
     for (long long b = 0; b < L.nblocks; b++) {
         acc += (L.tc2_goff[b + 1] - L.tc2_goff[b]) + (L.tc2_goff2[b + 1] - L.tc2_goff2[b]);
@@ -1690,12 +1714,13 @@ static size_t t2_flag_bytes(const Tc2Args &a)
 // bytes per VDF tile in an item slot: A hi, A lo, the FP32 side tile, the slot header
 static int t2_region(int P, int VB)
 {
-    return (2 * T2_ATILE + (TC_ROWS / VB) * P * VB * 4 + T2_HDR + 1023) / 1024 * 1024;
+    return (2 * t2_atile(P) + (TC_ROWS / VB) * P * VB * 4 + T2_HDR + 1023) / 1024 * 1024;
 }
 
-static size_t t2_smem(int region)
+static size_t t2_smem(int P, int region)
 {
-    return (size_t)T2_NSTW * T2_GREC + 4 * (size_t)region + (2 * T2_NSTW + 17) * sizeof(uint64_t) + 16;
+    return (size_t)t2_nstw(P) * t2_grec(P) + 2 * (size_t)t2_nslot(P) * region +
+           (2 * (t2_nstw(P) + t2_nslot(P) + t2_nacc(P)) + 5) * sizeof(uint64_t) + 16;
 }
 
 // the launch of a block-form kernel: one unit per CTA (grid = units), or
@@ -1706,7 +1731,7 @@ static int t2_launch(Ctx *c, const Tc2Launch &Lh, bool persistent, cudaStream_t 
 {
     const int total = Lh.ubase[Lh.ngrids];
     if (total <= 0) return DGV_OK;
-    const size_t smem = t2_smem(Lh.region);
+    const size_t smem = t2_smem(P, Lh.region);
     auto fn = k_collide_tc2<VB, P, MODE, MG>;
     DGV_CUDA(c, cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     if (!persistent) {
@@ -1860,7 +1885,7 @@ static int tc2_begin(Ctx *c, const double *d_f, int nvdf, Tc2Call &k, cudaStream
     const int VB = nvdf > 64 ? 128 : (nvdf > 32 ? 64 : 32), NDG = TC_ROWS / VB;
     const int nbt = (nvdf + VB - 1) / VB, NV = nbt * VB, ng = (g.Nc + NDG - 1) / NDG;
     const size_t fbytes = (size_t)nbt * g.Nc * g.P * VB * sizeof(float);
-    const size_t f16bytes = (size_t)nbt * 2 * g.Nc * VB * T2_K * 2;
+    const size_t f16bytes = (size_t)nbt * 2 * g.Nc * VB * t2_k(g.P) * 2;
     const size_t qbytes = (size_t)g.N * NV * sizeof(double);
     rc = ensure_buffer(c, &c->d_tcF, &c->tcF_bytes, fbytes + f16bytes + NV * sizeof(double));
     if (rc) return rc;
@@ -2178,10 +2203,10 @@ static int tc2_prepare_adjoint(Ctx *c)
     const long long nb = L.nblocks;
     L.tc2_goff2.assign((size_t)nb + 1, 0);
     for (long long b = 0; b < nb; b++)
-        L.tc2_goff2[b + 1] = L.tc2_goff2[b] + (__builtin_popcount(L.tc2_mask[nb + b]) * g.P + T2_N - 1) / T2_N;
+        L.tc2_goff2[b + 1] = L.tc2_goff2[b] + (__builtin_popcount(L.tc2_mask[nb + b]) * g.P + t2_n(g.P) - 1) / t2_n(g.P);
     unsigned *d_mask = nullptr;
     long long *d_goff = nullptr;
-    cudaError_t e = cudaMalloc(&L.tc2_Wv, (size_t)std::max<long long>(1, L.tc2_goff2[nb]) * T2_GREC);
+    cudaError_t e = cudaMalloc(&L.tc2_Wv, (size_t)std::max<long long>(1, L.tc2_goff2[nb]) * t2_grec(g.P));
     if (e != cudaSuccess || cudaMalloc(&d_mask, sizeof(unsigned) * std::max<long long>(1, nb)) != cudaSuccess ||
         cudaMalloc(&d_goff, sizeof(long long) * (nb + 1)) != cudaSuccess) {
         cudaGetLastError();
@@ -2222,7 +2247,7 @@ static int vjp_tc_body(Ctx *c, const double *d_f, const double *d_v, double *d_g
     const int VB = nvdf > 64 ? 128 : (nvdf > 32 ? 64 : 32), NDG = TC_ROWS / VB;
     const int nbt = (nvdf + VB - 1) / VB, NV = nbt * VB, ng = (g.Nc + NDG - 1) / NDG;
     const size_t fbytes = (size_t)nbt * g.Nc * g.P * VB * sizeof(float);
-    const size_t f16bytes = (size_t)nbt * 2 * g.Nc * VB * T2_K * 2;
+    const size_t f16bytes = (size_t)nbt * 2 * g.Nc * VB * t2_k(g.P) * 2;
     const size_t gbytes = (size_t)g.N * NV * sizeof(double);
     rc = ensure_buffer(c, &c->d_tcF, &c->tcF_bytes, 2 * fbytes + f16bytes + 2 * NV * sizeof(double));
     if (rc) return rc;
@@ -2371,13 +2396,13 @@ int tc_plan(Ctx *c, int nvdf, long long *launches, long long *items, double *flo
         tc2_sets(c);
         std::vector<int> first, count;
         if ((rc = tc_work_lists(c, NDG, 256 + NDG, L.tc2_sets, first, count, &tl, 1))) return rc;
-        // per item and VDF tile: 2 K steps x 3 split products over its issued columns
+        // per item and VDF tile: the K steps x 3 split products over its issued columns
         const long long cols = L.tc_list_work[256 + NDG];
         const int tpc = c->tc_tiles_per_cta;
         const bool uniform = nbt <= tpc || nbt % tpc == 0;
         *launches = c->tc_persistent && uniform ? 1 : (long long)L.tc2_sets.size() - 1;
         *items = L.tc_list_items[256 + NDG] * nbt;
-        *flop = (double)cols * nbt * 6.0 * 2.0 * TC_ROWS * 16;
+        *flop = (double)cols * nbt * 3.0 * 2.0 * TC_ROWS * t2_k(g.P);
     } else {
         if ((rc = tc_prepare(c))) return rc;
         if ((rc = tc_lists(c, NDG, &tl))) return rc;

@@ -40,9 +40,21 @@ __device__ __forceinline__ void fence_mbar_init()
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
 
+// HOLD: how long (ns) the hardware may hold the thread; 0: its own default
+template <uint32_t HOLD = 0>
 __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity)
 {
     uint32_t ok;
+    if constexpr (HOLD > 0) {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(smem_u32(bar)), "r"(parity), "r"(HOLD)
+            : "memory");
+        return ok != 0;
+    }
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
@@ -57,13 +69,14 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity)
 // waiting it also looks at the error flag about once a millisecond, so once
 // one wait has given up the other waits of the launch (and of launches queued
 // behind it) give up within a millisecond instead of each running its limit.
+template <uint32_t HOLD = 0>
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, int *err,
                                           unsigned long long limit_ns = WAIT_LIMIT_NS)
 {
-    if (mbar_try_wait(bar, parity)) return true;
+    if (mbar_try_wait<HOLD>(bar, parity)) return true;
     const unsigned long long t0 = globaltimer_ns();
     unsigned long long tcheck = t0;
-    while (!mbar_try_wait(bar, parity)) {
+    while (!mbar_try_wait<HOLD>(bar, parity)) {
         const unsigned long long t = globaltimer_ns();
         if (t - t0 > limit_ns) {
             *(volatile int *)err = 1;  // host-mapped flag, read after the stream synchronises
