@@ -280,7 +280,7 @@ int dgv_ctx_create(const dgv_grid_desc *desc, int device, dgv_ctx **out)
     double **dst[4] = {&c->d_nu, &c->d_nv, &c->d_nw, &c->d_nwt};
     const std::vector<double> *src[4] = {&g.nu, &g.nv, &g.nw, &g.nwt};
     for (int k = 0; k < 4; k++) {
-        if (cudaMalloc(dst[k], nb) != cudaSuccess || cudaMemcpy(*dst[k], src[k]->data(), nb, cudaMemcpyHostToDevice) != cudaSuccess) {
+        if (cudaMalloc(dst[k], nb) != cudaSuccess || upload(*dst[k], src[k]->data(), nb) != cudaSuccess) {
             cudaGetLastError();
             destroy_ctx(c);
             delete h;

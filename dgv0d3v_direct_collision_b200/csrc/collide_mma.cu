@@ -684,8 +684,8 @@ static int mma_boxes(Ctx *c, MmaList &M, bool across)
     void *d = nullptr, *e = nullptr;
     cudaError_t rc = cudaMalloc(&d, std::max<size_t>(1, seg.size()) * sizeof(unsigned long long));
     if (rc == cudaSuccess) rc = cudaMalloc(&e, sfirst.size() * sizeof(int));
-    if (rc == cudaSuccess) rc = cudaMemcpy(d, seg.data(), seg.size() * sizeof(unsigned long long), cudaMemcpyHostToDevice);
-    if (rc == cudaSuccess) rc = cudaMemcpy(e, sfirst.data(), sfirst.size() * sizeof(int), cudaMemcpyHostToDevice);
+    if (rc == cudaSuccess) rc = upload(d, seg.data(), seg.size() * sizeof(unsigned long long));
+    if (rc == cudaSuccess) rc = upload(e, sfirst.data(), sfirst.size() * sizeof(int));
     if (rc != cudaSuccess) {
         cudaGetLastError();
         cudaFree(d);
@@ -751,7 +751,7 @@ static int mma_plan(Ctx *c, MmaList &M, const MmaShape &S, int cell0, int cell1,
     }
     pl.nunits = (int)units.size();
     DGV_CUDA(c, cudaMalloc(&pl.units, std::max<size_t>(1, units.size()) * sizeof(MmaUnit)));
-    const cudaError_t e = cudaMemcpy(pl.units, units.data(), units.size() * sizeof(MmaUnit), cudaMemcpyHostToDevice);
+    const cudaError_t e = upload(pl.units, units.data(), units.size() * sizeof(MmaUnit));
     if (e != cudaSuccess) {
         cudaFree(pl.units);
         return set_err(c, DGV_ECUDA, std::string("collide plan: ") + cudaGetErrorString(e));
@@ -778,7 +778,7 @@ static int mma_bounds(Ctx *c, MmaPlan *pl, int nchunks, const int2 **out)
     }
     void *d = nullptr;
     DGV_CUDA(c, cudaMalloc(&d, sizeof(int2) * b.size()));
-    const cudaError_t e = cudaMemcpy(d, b.data(), sizeof(int2) * b.size(), cudaMemcpyHostToDevice);
+    const cudaError_t e = upload(d, b.data(), sizeof(int2) * b.size());
     if (e != cudaSuccess) {
         cudaFree(d);
         return set_err(c, DGV_ECUDA, std::string("collide plan: ") + cudaGetErrorString(e));

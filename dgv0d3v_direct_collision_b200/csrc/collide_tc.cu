@@ -622,7 +622,7 @@ static int tc_prepare(Ctx *c)
     int rc = tc_value_scale(c, &L.tc_vscale);
     if (rc) return rc;
     DGV_CUDA(c, cudaMalloc(&L.tc_chunk_start, sizeof(int) * (L.nblocks + 1)));
-    DGV_CUDA(c, cudaMemcpy(L.tc_chunk_start, cs.data(), sizeof(int) * (L.nblocks + 1), cudaMemcpyHostToDevice));
+    DGV_CUDA(c, upload(L.tc_chunk_start, cs.data(), sizeof(int) * (L.nblocks + 1)));
     DGV_CUDA(c, cudaMalloc(&L.tc_V, (size_t)std::max<long long>(1, nch) * TC_REC));
     if (L.nblocks)
         k_tc_build<<<(unsigned)L.nblocks, 256, 0, c->stream>>>(L.blk, (const double *)L.rows64, L.RD64,
@@ -758,9 +758,9 @@ static int tc_work_lists(Ctx *c, int NDG, int key, const std::vector<int> &sets,
     DGV_CUDA(c, cudaMalloc(&d[0], sizeof(TcItem) * std::max<size_t>(1, items.size())));
     DGV_CUDA(c, cudaMalloc(&d[1], sizeof(int) * start.size()));
     DGV_CUDA(c, cudaMalloc(&d[2], sizeof(int) * tile_of.size()));
-    if (!items.empty()) DGV_CUDA(c, cudaMemcpy(d[0], items.data(), sizeof(TcItem) * items.size(), cudaMemcpyHostToDevice));
-    DGV_CUDA(c, cudaMemcpy(d[1], start.data(), sizeof(int) * start.size(), cudaMemcpyHostToDevice));
-    DGV_CUDA(c, cudaMemcpy(d[2], tile_of.data(), sizeof(int) * tile_of.size(), cudaMemcpyHostToDevice));
+    if (!items.empty()) DGV_CUDA(c, upload(d[0], items.data(), sizeof(TcItem) * items.size()));
+    DGV_CUDA(c, upload(d[1], start.data(), sizeof(int) * start.size()));
+    DGV_CUDA(c, upload(d[2], tile_of.data(), sizeof(int) * tile_of.size()));
     L.tc_lists[key] = {d[0], d[1], d[2]};
     L.tc_list_work[key] = wsum;
     L.tc_list_items[key] = (long long)items.size();

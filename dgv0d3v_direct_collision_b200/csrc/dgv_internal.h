@@ -219,6 +219,11 @@ int set_err(Ctx *c, int code, const std::string &msg);
                                 std::string(#call) + ": " + cudaGetErrorString(e_)); \
     } while (0)
 
+// Host data into a device array that no queued work uses; returns when it has
+// arrived.  A cudaMemcpy from pageable memory may return with the data only
+// staged, and streams made with cudaStreamNonBlocking (the contexts' own, and
+// most callers') do not wait for the stream it runs on.
+cudaError_t upload(void *dst, const void *src, size_t bytes);
 int ensure_buffer(Ctx *c, double **p, size_t *have, size_t need_bytes);
 // frees the layouts of a DGV_LAYOUT_* mask (rebuilt on their next use)
 int release_layouts(Ctx *c, int mask);

@@ -20,6 +20,13 @@
 
 namespace dgv {
 
+// On the legacy stream, as cudaMemcpy: the caller's stream may be captured.
+cudaError_t upload(void *dst, const void *src, size_t bytes)
+{
+    const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, cudaStreamLegacy);
+    return e == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : e;
+}
+
 void free_layout(Layout &L)
 {
     if (L.blk) cudaFree(L.blk);
@@ -155,9 +162,9 @@ static int upload_layout(Ctx *c, std::vector<BlockInfo> &blk, std::vector<double
     DGV_CUDA(c, cudaMalloc(&L.blk, bb));
     DGV_CUDA(c, cudaMalloc(&L.rows64, r64));
     DGV_CUDA(c, cudaMalloc(&L.rows32, r32));
-    if (!blk.empty()) DGV_CUDA(c, cudaMemcpy(L.blk, blk.data(), blk.size() * sizeof(BlockInfo), cudaMemcpyHostToDevice));
-    if (!rows64.empty()) DGV_CUDA(c, cudaMemcpy(L.rows64, rows64.data(), rows64.size() * sizeof(double), cudaMemcpyHostToDevice));
-    if (!rows32.empty()) DGV_CUDA(c, cudaMemcpy(L.rows32, rows32.data(), rows32.size() * sizeof(float), cudaMemcpyHostToDevice));
+    if (!blk.empty()) DGV_CUDA(c, upload(L.blk, blk.data(), blk.size() * sizeof(BlockInfo)));
+    if (!rows64.empty()) DGV_CUDA(c, upload(L.rows64, rows64.data(), rows64.size() * sizeof(double)));
+    if (!rows32.empty()) DGV_CUDA(c, upload(L.rows32, rows32.data(), rows32.size() * sizeof(float)));
     return DGV_OK;
 }
 
@@ -289,7 +296,7 @@ int get_chunks(Ctx *c, int nchunks, int **d_bounds)
     }
     int *d = nullptr;
     DGV_CUDA(c, cudaMalloc(&d, sizeof(int) * (nchunks + 1)));
-    DGV_CUDA(c, cudaMemcpy(d, bounds.data(), sizeof(int) * (nchunks + 1), cudaMemcpyHostToDevice));
+    DGV_CUDA(c, upload(d, bounds.data(), sizeof(int) * (nchunks + 1)));
     L.chunks[nchunks] = d;
     *d_bounds = d;
     return DGV_OK;
