@@ -278,10 +278,12 @@ extern "C" int dgv_write_A_file(dgv_ctx *ctx, const char *path, int64_t max_subr
 
 namespace {
 
-// f may live on the host or the device: cudaMemcpyDefault infers the direction
-std::string copy_any(double *dst, const double *src, size_t n)
+// f may live on the host or the device: cudaMemcpyDefault infers the direction.
+// On the context's stream: after the work queued there, and complete on return.
+std::string copy_any(Ctx *c, double *dst, const double *src, size_t n)
 {
-    cudaError_t e = cudaMemcpy(dst, src, n * sizeof(double), cudaMemcpyDefault);
+    cudaError_t e = cudaMemcpyAsync(dst, src, n * sizeof(double), cudaMemcpyDefault, c->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     return e == cudaSuccess ? "" : cudaGetErrorString(e);
 }
 
@@ -374,7 +376,7 @@ extern "C" int dgv_write_solution(dgv_ctx *ctx, const char *path, const double *
     const int rkmts = order > 0 ? order : 1;
     // f1..f4 are written as zeros: the multistep formulas never read them
     std::vector<double> fh(N), prev((size_t)(rkmts - 1) * N, 0.0);
-    std::string e = copy_any(fh.data(), f, N);
+    std::string e = copy_any(c, fh.data(), f, N);
     if (!e.empty()) return set_err(c, DGV_ECUDA, "write_solution: " + e);
     e = write_sol(path, (int32_t)N, rkmts, e_time, dt,
                   {{fh.data(), N * sizeof(double)},
@@ -396,7 +398,7 @@ extern "C" int dgv_read_solution(dgv_ctx *ctx, const char *path, double *f, doub
     const size_t N = (size_t)c->grid.N;
     if ((size_t)s.N != N) return set_err(c, DGV_EINVAL, "read_solution: array length differs from the grid's N");
     const double *arr = reinterpret_cast<const double *>(s.arrays.data());
-    e = copy_any(f, arr, N);
+    e = copy_any(c, f, arr, N);
     if (!e.empty()) return set_err(c, DGV_ECUDA, "read_solution: " + e);
     int rc = ab_history_set(c, s.rkmts, arr + (size_t)s.rkmts * N);  // after f, f1..f(rkmts-1)
     if (rc) return rc;

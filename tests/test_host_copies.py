@@ -167,3 +167,8 @@ def test_device_sources_upload_the_same_way():
         src = re.sub(r"//[^\n]*", "", open(path).read())
         calls = re.findall(r"cudaMemcpy(?:2D|ToSymbol)?\([^;]*;", src)
         assert all("cudaMemcpyHostToDevice" not in c for c in calls), (os.path.basename(path), calls)
+
+
+def test_solution_files_are_in_stream_order(harness, tmp_path):
+    r = subprocess.run([harness, "solution", str(tmp_path / "f.sol")], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout
