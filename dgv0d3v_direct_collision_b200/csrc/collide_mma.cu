@@ -705,12 +705,52 @@ struct MmaShape {
     int c_tile, c_stage, c_unit, c_flush;  // costs (SM cycles, fitted): stage per tile, stage, unit, its end per tile
 };
 
+// Plans of slices of the output cells kept per list, the least recently used
+// given up: a rank has one slice, a caller may walk through all Nc^2 / 2.  (A
+// plan is 32 bytes per box on the device, 0.3 MB at 27^3, and a pass over the
+// boxes to build.)  The whole grid's plan stays, which captured steps hold, and
+// so do the plans that a caller's capture has recorded.
+constexpr int MMA_SLICES = 64;
+
+static int mma_make_room(Ctx *c, MmaList &M)
+{
+    for (;;) {
+        auto old = M.plans.end();
+        int n = 0;
+        for (auto it = M.plans.begin(); it != M.plans.end(); ++it) {
+            if (it->second.captured || it->first == std::make_pair(0, c->grid.Nc)) continue;
+            n++;
+            if (old == M.plans.end() || it->second.used < old->second.used) old = it;
+        }
+        if (n < MMA_SLICES) return DGV_OK;
+        DGV_CUDA(c, cudaStreamSynchronize(c->stream));  // launches that read it
+        free_plan(old->second);
+        M.plans.erase(old);
+    }
+}
+
 static int mma_plan(Ctx *c, MmaList &M, const MmaShape &S, int cell0, int cell1, MmaPlan **out)
 {
     const Grid &g = c->grid;
     const std::pair<int, int> key(cell0, cell1);
+    bool captured = false;
+    if (key != std::make_pair(0, g.Nc)) {
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(c->stream, &st) != cudaSuccess) cudaGetLastError();
+        captured = st != cudaStreamCaptureStatusNone;
+    }
+    M.clock++;
     auto it = M.plans.find(key);
-    if (it != M.plans.end()) { *out = &it->second; return DGV_OK; }
+    if (it != M.plans.end()) {
+        it->second.used = M.clock;
+        it->second.captured |= captured;
+        *out = &it->second;
+        return DGV_OK;
+    }
+    if (!captured) {
+        const int rc = mma_make_room(c, M);
+        if (rc) return rc;
+    }
     std::vector<MmaUnit> units;
     MmaPlan pl;
     pl.cost.push_back(0);
@@ -750,6 +790,8 @@ static int mma_plan(Ctx *c, MmaList &M, const MmaShape &S, int cell0, int cell1,
         }
     }
     pl.nunits = (int)units.size();
+    pl.used = M.clock;
+    pl.captured = captured;
     DGV_CUDA(c, cudaMalloc(&pl.units, std::max<size_t>(1, units.size()) * sizeof(MmaUnit)));
     const cudaError_t e = upload(pl.units, units.data(), units.size() * sizeof(MmaUnit));
     if (e != cudaSuccess) {

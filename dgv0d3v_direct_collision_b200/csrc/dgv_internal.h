@@ -60,6 +60,8 @@ struct MmaPlan {
     std::vector<long long> cost;
     std::vector<int> first, last, per_stage;
     std::map<int, void *> bounds;
+    unsigned long long used = 0;  // MmaList::clock at its last use
+    bool captured = false;        // a caller's graph may hold its arrays
 };
 
 // Stages of the layout's pairs in box order (collide_mma.cu; device arrays),
@@ -68,7 +70,9 @@ struct MmaList {
     void *segs = nullptr, *sfirst = nullptr;
     std::vector<MmaBox> box;
     std::map<std::pair<int, int>, MmaPlan> plans;
+    unsigned long long clock = 0;
 };
+void free_plan(MmaPlan &pl);
 
 // Device copy of the A-arrays in the pair layout.
 //   rows64[pair] = { int32 o1, int32 o2, double v[P], pad }  (RD64 doubles)

@@ -27,6 +27,12 @@ cudaError_t upload(void *dst, const void *src, size_t bytes)
     return e == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : e;
 }
 
+void free_plan(MmaPlan &pl)
+{
+    if (pl.units) cudaFree(pl.units);
+    for (auto &b : pl.bounds) cudaFree(b.second);
+}
+
 void free_layout(Layout &L)
 {
     if (L.blk) cudaFree(L.blk);
@@ -36,10 +42,7 @@ void free_layout(Layout &L)
     for (MmaList *m : {&L.mma, &L.groups}) {
         if (m->segs) cudaFree(m->segs);
         if (m->sfirst) cudaFree(m->sfirst);
-        for (auto &kv : m->plans) {
-            if (kv.second.units) cudaFree(kv.second.units);
-            for (auto &b : kv.second.bounds) cudaFree(b.second);
-        }
+        for (auto &kv : m->plans) free_plan(kv.second);
     }
     for (void *p : {L.vjp_first, L.vjp_tiles, L.vjp_items})
         if (p) cudaFree(p);
