@@ -33,17 +33,22 @@ void free_plan(MmaPlan &pl)
     for (auto &b : pl.bounds) cudaFree(b.second);
 }
 
+static void free_list(MmaList &m)
+{
+    if (m.segs) cudaFree(m.segs);
+    if (m.sfirst) cudaFree(m.sfirst);
+    for (auto &kv : m.plans) free_plan(kv.second);
+    m = MmaList();
+}
+
 void free_layout(Layout &L)
 {
     if (L.blk) cudaFree(L.blk);
     if (L.rows64) cudaFree(L.rows64);
     if (L.rows32) cudaFree(L.rows32);
     for (auto &kv : L.chunks) cudaFree(kv.second);
-    for (MmaList *m : {&L.mma, &L.groups}) {
-        if (m->segs) cudaFree(m->segs);
-        if (m->sfirst) cudaFree(m->sfirst);
-        for (auto &kv : m->plans) free_plan(kv.second);
-    }
+    free_list(L.mma);
+    free_list(L.groups);
     for (void *p : {L.vjp_first, L.vjp_tiles, L.vjp_items})
         if (p) cudaFree(p);
     if (L.tc_V) cudaFree(L.tc_V);
@@ -76,9 +81,10 @@ int release_layouts(Ctx *c, int mask)
             }
         }
     };
-    if ((mask & DGV_LAYOUT_F32) && L.rows32) {
-        cudaFree(L.rows32);
+    if (mask & DGV_LAYOUT_F32) {
+        if (L.rows32) cudaFree(L.rows32);
         L.rows32 = nullptr;
+        free_list(L.groups);
     }
     if (mask & DGV_LAYOUT_TC_CHUNK) {
         if (L.tc_V) cudaFree(L.tc_V);

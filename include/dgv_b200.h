@@ -94,7 +94,8 @@ extern "C" {
                                  /* returns DGV_ETIMEOUT; resets itself       */
 
 /* layouts for dgv_release_layouts */
-#define DGV_LAYOUT_F32 1      /* FP32 rows of the pair layout (FP32-compensated Q) */
+#define DGV_LAYOUT_F32 1      /* FP32 rows of the pair layout (FP32-compensated Q) and */
+                              /* the work lists of their groups                 */
 #define DGV_LAYOUT_TC_CHUNK 2 /* records of the tensor-core chunk form          */
 #define DGV_LAYOUT_TC_BLOCK 4 /* records of the block form and of its adjoint   */
 #define DGV_LAYOUT_TC_ADJ 8   /* only the adjoint's second record set           */

@@ -137,20 +137,23 @@ int main(int, char **argv)
 """
 
 
-@pytest.fixture(scope="module")
-def harness(tmp_path_factory):
+def build_harness(d, text):
     cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
     cxx = shutil.which("g++")
     if not cxx or not os.path.exists(os.path.join(cuda, "include", "cuda_runtime.h")):
         pytest.skip("needs g++ and the CUDA headers")
-    d = tmp_path_factory.mktemp("host_copies")
     src = d / "harness.cpp"
-    src.write_text(HARNESS)
+    src.write_text(text)
     exe = d / "harness"
     subprocess.check_call([cxx, "-std=c++17", "-O1", "-I", os.path.join(cuda, "include"), "-I", os.path.join(ROOT, "include"),
                            "-I", CSRC, str(src)] + [os.path.join(CSRC, f) for f in ("layout.cpp", "afile.cpp", "grid.cpp")] +
                           ["-o", str(exe)])
     return str(exe)
+
+
+@pytest.fixture(scope="module")
+def harness(tmp_path_factory):
+    return build_harness(tmp_path_factory.mktemp("host_copies"), HARNESS)
 
 
 @pytest.mark.parametrize("what", ["layout", "chunks"])
