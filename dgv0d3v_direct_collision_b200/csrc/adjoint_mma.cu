@@ -341,15 +341,33 @@ static int vjp_prepare(Ctx *c)
     return DGV_OK;
 }
 
+// Scratch of one launch at most: 2 N doubles per VDF are 426 VDFs at 27^3,
+// seconds of work, beside which another launch's start is nothing
+constexpr long long VJ_SCRATCH = 128LL << 20;
+
+static int vjp_mma_launch(Ctx *c, const double *d_f, const double *d_v, double *d_g, int nvdf);
+
 int vjp_mma_device(Ctx *c, const double *d_f, const double *d_v, double *d_g, int nvdf)
 {
     if (!c->lay.blk) return set_err(c, DGV_ESTATE, "vjp: no A-arrays loaded");
     const Grid &g = c->grid;
-    Layout &L = c->lay;
     if (g.N > INT32_MAX / 2) return set_err(c, DGV_EUNSUP, "vjp: grid too large");
     int rc = vjp_prepare(c);
     if (rc) return rc;
     if ((rc = ensure_errflag(c))) return rc;
+    const long long most = std::max<long long>(1, VJ_SCRATCH / (16 * g.N));
+    for (long long v = 0; v < nvdf; v += most) {
+        const long long at = v * g.N;
+        if ((rc = vjp_mma_launch(c, d_f + at, d_v + at, d_g + at, (int)std::min(most, nvdf - v)))) return rc;
+    }
+    return DGV_OK;
+}
+
+static int vjp_mma_launch(Ctx *c, const double *d_f, const double *d_v, double *d_g, int nvdf)
+{
+    const Grid &g = c->grid;
+    const Layout &L = c->lay;
+    int rc;
     const long long n = (long long)nvdf * g.N;
     // the sums (f, v and g of the caller may be one array), the item counter, c
     if ((rc = ensure_buffer(c, &c->d_glm, &c->glm_bytes, sizeof(double) * (size_t)(2 * n + 1)))) return rc;
