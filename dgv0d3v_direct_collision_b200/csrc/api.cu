@@ -273,6 +273,7 @@ int dgv_ctx_create(const dgv_grid_desc *desc, int device, dgv_ctx **out)
     if (rc) { delete h; return rc; }
     rc = gram_inverse(c);
     if (rc) { delete h; return rc; }
+    c->tc_set_mb = tc_default_set_mb(c->grid.P);
     if (cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking) != cudaSuccess) { delete h; return DGV_ECUDA; }
     c->stream = c->own_stream;
     const Grid &g = c->grid;
@@ -375,7 +376,7 @@ int dgv_set_option(dgv_ctx *ctx, int option, int64_t value)
             ctx->c.tc_tuned_adj.clear();
             if (!ctx->c.tc_user_launch) {
                 ctx->c.tc_tiles_per_cta = 2;
-                ctx->c.tc_set_mb = 48;
+                ctx->c.tc_set_mb = tc_default_set_mb(ctx->c.grid.P);
                 ctx->c.tc_persistent = 0;
             }
         }

@@ -826,7 +826,6 @@ __host__ __device__ constexpr int t2_atile(int P) { return TC_ROWS * t2_k(P) * 2
 __host__ __device__ constexpr int t2_nstw(int P) { return P == 8 ? 8 : 3; }        // W ring stages
 __host__ __device__ constexpr int t2_nslot(int P) { return P == 8 ? 4 : 2; }       // item slots
 __host__ __device__ constexpr int t2_nacc(int P) { return 512 / t2_n(P); }         // accumulators in tensor memory
-constexpr int T2_SETREC = 32 * 1024;  // bytes that a column group counts in the size of a block set, whatever P
 constexpr int T2_EPI_WARPS = 8;
 // slot header, after the side tile of the slot's first VDF tile: the item's
 // column count, for each rank jj of its mask the offset (floats) l*VB of the
@@ -1650,7 +1649,7 @@ static void tc2_sets(Ctx *c)
     // about tc_set_mb MB of the collision operator's (compacted) records per set
     L.tc2_sets.clear();
     L.tc2_sets.push_back(0);
-    const long long per_set = std::max<long long>(1, ((long long)c->tc_set_mb << 20) / T2_SETREC);
+    const long long per_set = std::max<long long>(1, ((long long)c->tc_set_mb << 20) / t2_grec(c->grid.P));
     long long acc = 0;
     for (long long b = 0; b < L.nblocks; b++) {
         acc += L.tc2_goff[b + 1] - L.tc2_goff[b];
@@ -1673,7 +1672,7 @@ static void tc2_sets_adjoint(Ctx *c)
     Layout &L = c->lay;
     if (!L.tc2_sets_adj.empty()) return;
     L.tc2_sets_adj.push_back(0);
-    const long long per_set = std::max<long long>(1, ((long long)c->tc_set_mb << 20) / T2_SETREC);
+    const long long per_set = std::max<long long>(1, ((long long)c->tc_set_mb << 20) / t2_grec(c->grid.P));
     long long acc = 0;
     for (long long b = 0; b < L.nblocks; b++) {
         acc += (L.tc2_goff[b + 1] - L.tc2_goff[b]) + (L.tc2_goff2[b + 1] - L.tc2_goff2[b]);
@@ -2076,8 +2075,11 @@ static int tc2_autotune(Ctx *c, const double *d_f, double *d_q, int nvdf, double
     // records per launch up to 48 MB: with the f tiles and the FP64
     // accumulators a launch touches (~84 MB at 27^3 x 256), its working set
     // then (nearly) stays in the 126 MB L2; 96 MB sets ran as fast but read
-    // their records ~10x from DRAM (measured)
-    const int tiles[2] = {2, 1}, mbs[2] = {24, 48};
+    // their records ~10x from DRAM (measured).  Eight nodes per cell have 4 KB
+    // a block: 3 and 6 MB are as many blocks, and a persistent launch needs
+    // several sets for its CTAs to share (150 VDFs, 14^3: 18.9 / 19.1 ms with
+    // 3 / 6 MB, 20.9 / 23.0 with 24 / 48; 20^3: 326 / 324, 322 / 321)
+    const int most = tc_default_set_mb(c->grid.P), tiles[2] = {2, 1}, mbs[2] = {most / 2, most};
     float best_ms = 1e30f;
     Ctx::TcChoice best{c->tc_tiles_per_cta, c->tc_set_mb, c->tc_persistent};
     int rc = DGV_OK;

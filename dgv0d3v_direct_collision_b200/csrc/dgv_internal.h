@@ -182,7 +182,7 @@ struct Ctx {
     bool ktiming = false;
     int tc_form = 2;  // DGV_OPT_TCFORM: 1 chunk form, 2 block form (8 or 27 nodes per cell)
     int tc_tiles_per_cta = 2;  // DGV_OPT_TCTILES: VDF tiles per CTA in the block form
-    int tc_set_mb = 48;        // DGV_OPT_TCSETMB: block form, MB of records per launch
+    int tc_set_mb = 48;        // DGV_OPT_TCSETMB: block form, MB of records per launch (tc_default_set_mb)
     long long wait_limit_us = 0;  // DGV_OPT_WAIT_LIMIT_US: bounded waits of the block form (0 = 4 s)
     int f_global = 0;             // DGV_OPT_FGLOBAL: 1 = CUDA-core kernels gather f from global memory
     bool tc_autotune = true;      // DGV_OPT_TCAUTOTUNE: tune tiles per CTA and records per launch
@@ -228,6 +228,8 @@ int set_err(Ctx *c, int code, const std::string &msg);
 // staged, and streams made with cudaStreamNonBlocking (the contexts' own, and
 // most callers') do not wait for the stream it runs on.
 cudaError_t upload(void *dst, const void *src, size_t bytes);
+// block form: MB of records per launch unless the caller or the tuning chose
+inline int tc_default_set_mb(int P) { return P == 8 ? 6 : 48; }
 int ensure_buffer(Ctx *c, double **p, size_t *have, size_t need_bytes);
 // frees the layouts of a DGV_LAYOUT_* mask (rebuilt on their next use)
 int release_layouts(Ctx *c, int mask);

@@ -63,8 +63,9 @@ extern "C" {
                            /* read from L2 per 256 rows, one accumulator per  */
                            /* tile) or 1 (two accumulators per tile)          */
 #define DGV_OPT_TCSETMB 6  /* block form: MB of block records per kernel     */
-                           /* launch (default 48; a launch's records are read */
-                           /* by all its CTAs, so they should stay in L2)     */
+                           /* launch (default 48, with 8 nodes per cell 6; a  */
+                           /* launch's records are read by all its CTAs, so   */
+                           /* they should stay in L2)                         */
 #define DGV_OPT_WAIT_LIMIT_US 7  /* microseconds after which a bounded wait   */
                                  /* of a collision kernel (block form, FP64,  */
                                  /* FP32-compensated, mixed terms, adjoint)   */
