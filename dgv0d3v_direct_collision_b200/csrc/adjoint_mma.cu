@@ -61,6 +61,7 @@ struct VjpMmaArgs {
     int *err;
     long long N, nitems, total;
     int Nc, Mv, Mw, ccell, rowb;
+    int withhold;    // test: the first tile of the first item is not copied
     unsigned magic;  // x = l * Nc -> l = high word of x * magic (Nc > 1)
     unsigned long long wait_ns;
 };
@@ -113,9 +114,9 @@ __global__ void __launch_bounds__(32 * VJ_WARPS, 1) k_vjp_mma(const __grid_const
         for (int t = lane; t < nt; t += 32) tl[t] = __ldg(a.tiles + t0 + t);
         __syncwarp();
         int sent = 0, sslot = slot;
-        auto send = [&]() {  // the next tile's rows into the ring
+        auto send = [&](bool hold = false) {  // the next tile's rows into the ring
             if (sent >= nt) return;
-            if (lane == 0) {
+            if (lane == 0 && !hold) {
                 const unsigned x = tl[sent];
                 const int n = (int)(x >> 10 & 15u);
                 mbar_arrive_expect_tx(&full[sslot], (uint32_t)(n * a.rowb));
@@ -125,7 +126,7 @@ __global__ void __launch_bounds__(32 * VJ_WARPS, 1) k_vjp_mma(const __grid_const
             sent++;
             sslot = sslot + 1 == VJ_NST ? 0 : sslot + 1;
         };
-        for (int s = 0; s < VJ_NST; s++) send();
+        for (int s = 0; s < VJ_NST; s++) send(a.withhold && id == 0 && s == 0);
         // rows: lane l has the cell of row l
         int D = 0;
         {
@@ -386,6 +387,8 @@ static int vjp_mma_launch(Ctx *c, const double *d_f, const double *d_v, double *
     a.Nc = g.Nc; a.Mv = g.d.Mv; a.Mw = g.d.Mw; a.ccell = g.ccell; a.rowb = L.RD64 * 8;
     a.magic = g.Nc > 1 ? (unsigned)((1ULL << 32) / (unsigned)g.Nc + 1) : 0u;
     a.wait_ns = wait_limit_ns(c);
+    a.withhold = c->test_withhold ? 1 : 0;
+    c->test_withhold = false;
     const size_t smem = (size_t)VJ_WARPS * vjp_warp_bytes(g.P, a.rowb);
     auto fn = g.P == 27 ? k_vjp_mma<27> : k_vjp_mma<8>;
     DGV_CUDA(c, cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

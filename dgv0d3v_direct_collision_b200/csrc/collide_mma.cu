@@ -82,6 +82,7 @@ struct MmaArgs {
     int Nc, Mv, Mw, nchunks, cell0, ncell, rowb, nst;
     int part_smem, red_tiles;
     int off_f, off_g, off_part, off_red, off_bar;  // shared-memory layout (bytes)
+    int withhold;  // test: the launch's first stage is not copied
     unsigned long long wait_ns;
 };
 
@@ -180,7 +181,8 @@ struct MmaFetch {
         pw.enter(a, b0, b1, warp);
         advance(a);
         advance(a);
-        for (int s = 0; s < a.nst; s++) issue(a);
+        const bool held = a.withhold && blockIdx.x == 0 && blockIdx.y == 0 && warp == 0;
+        for (int s = 0; s < a.nst; s++) issue(a, held && s == 0);
     }
     __device__ __forceinline__ void advance(const MmaArgs &a)
     {
@@ -194,16 +196,16 @@ struct MmaFetch {
             pw.next(a, b0, b1, warp);
         }
     }
-    __device__ __forceinline__ void issue(const MmaArgs &a)
+    __device__ __forceinline__ void issue(const MmaArgs &a, bool hold = false)
     {
         if (!have) return;
         const int off = (int)(ent >> 8 & 255ULL), len = (int)(ent & 255ULL);
         const int n = __shfl_sync(0xffffffffu, off + len, nseg - 1);
-        if (lane == 0) {
+        if (lane == 0 && !hold) {
             cnt[islot] = n;
             mbar_arrive_expect_tx(&full[islot], (uint32_t)(n * a.rowb));
         }
-        if (lane < nseg)
+        if (lane < nseg && !hold)
             bulk_g2s(ring + (islot * MM_SP + off) * a.rowb, a.rows + (size_t)(ent >> 16) * a.rowb,
                      (uint32_t)(len * a.rowb), &full[islot]);
         inflight++;
@@ -927,6 +929,8 @@ int collide_mma_device(Ctx *c, const double *d_f, const double *d_g, double *d_q
     a.units = (const MmaUnit *)pl->units; a.bounds = bounds;
     a.err = c->d_err; a.N = g.N; a.Nc = g.Nc; a.Mv = g.d.Mv; a.Mw = g.d.Mw; a.nchunks = nchunks;
     a.cell0 = cell0; a.ncell = cell1 - cell0; a.wait_ns = wait_limit_ns(c);
+    a.withhold = c->test_withhold ? 1 : 0;
+    c->test_withhold = false;
     MmaFn fn = g.P == 27 ? mma_pick<27>(f32, bil, gf) : mma_pick<8>(f32, bil, gf);
     DGV_CUDA(c, cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     KTimer kt(c);

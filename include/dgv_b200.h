@@ -90,9 +90,12 @@ extern "C" {
                                  /* copy in global memory (L1/L2); 1 = always */
                                  /* the global copy                           */
 #define DGV_OPT_TEST_WITHHOLD 8  /* 1: test of the bounded waits: the next    */
-                                 /* block-form call leaves one of its copies  */
-                                 /* unissued, so its waits run out and it     */
-                                 /* returns DGV_ETIMEOUT; resets itself       */
+                                 /* call on a grid of 8 or 27 nodes per cell  */
+                                 /* (tensor cores in the block form, FP64,    */
+                                 /* FP32-compensated, mixed terms, adjoint)   */
+                                 /* leaves one of its copies unissued, so its */
+                                 /* waits run out and it returns              */
+                                 /* DGV_ETIMEOUT; resets itself               */
 
 /* layouts for dgv_release_layouts */
 #define DGV_LAYOUT_F32 1      /* FP32 rows of the pair layout (FP32-compensated Q) and */
