@@ -61,7 +61,7 @@ struct VjpMmaArgs {
     int *err;
     long long N, nitems, total;
     int Nc, Mv, Mw, ccell, rowb;
-    int withhold;    // test: the first tile of the first item is not copied
+    int withhold;    // test: 1 = the tiles' barriers wait for an arrival that does not come
     unsigned magic;  // x = l * Nc -> l = high word of x * magic (Nc > 1)
     unsigned long long wait_ns;
 };
@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(32 * VJ_WARPS, 1) k_vjp_mma(const __grid_const
     unsigned *tl = reinterpret_cast<unsigned *>(G2 + VJP_ALIGN(P * VJ_S * 8) / 8);
     uint64_t *full = reinterpret_cast<uint64_t *>(tl + VJ_MAXT);
     if (lane == 0) {
-        for (int s = 0; s < VJ_NST; s++) mbar_init(&full[s], 1);
+        for (int s = 0; s < VJ_NST; s++) mbar_init(&full[s], 1 + a.withhold);
         fence_mbar_init();
     }
     __syncwarp();
@@ -114,9 +114,9 @@ __global__ void __launch_bounds__(32 * VJ_WARPS, 1) k_vjp_mma(const __grid_const
         for (int t = lane; t < nt; t += 32) tl[t] = __ldg(a.tiles + t0 + t);
         __syncwarp();
         int sent = 0, sslot = slot;
-        auto send = [&](bool hold = false) {  // the next tile's rows into the ring
+        auto send = [&]() {  // the next tile's rows into the ring
             if (sent >= nt) return;
-            if (lane == 0 && !hold) {
+            if (lane == 0) {
                 const unsigned x = tl[sent];
                 const int n = (int)(x >> 10 & 15u);
                 mbar_arrive_expect_tx(&full[sslot], (uint32_t)(n * a.rowb));
@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(32 * VJ_WARPS, 1) k_vjp_mma(const __grid_const
             sent++;
             sslot = sslot + 1 == VJ_NST ? 0 : sslot + 1;
         };
-        for (int s = 0; s < VJ_NST; s++) send(a.withhold && id == 0 && s == 0);
+        for (int s = 0; s < VJ_NST; s++) send();
         // rows: lane l has the cell of row l
         int D = 0;
         {

@@ -82,7 +82,6 @@ struct MmaArgs {
     int Nc, Mv, Mw, nchunks, cell0, ncell, rowb, nst;
     int part_smem, red_tiles;
     int off_f, off_g, off_part, off_red, off_bar;  // shared-memory layout (bytes)
-    int withhold;  // test: the launch's first stage is not copied
     unsigned long long wait_ns;
 };
 
@@ -181,8 +180,7 @@ struct MmaFetch {
         pw.enter(a, b0, b1, warp);
         advance(a);
         advance(a);
-        const bool held = a.withhold && blockIdx.x == 0 && blockIdx.y == 0 && warp == 0;
-        for (int s = 0; s < a.nst; s++) issue(a, held && s == 0);
+        for (int s = 0; s < a.nst; s++) issue(a);
     }
     __device__ __forceinline__ void advance(const MmaArgs &a)
     {
@@ -196,16 +194,16 @@ struct MmaFetch {
             pw.next(a, b0, b1, warp);
         }
     }
-    __device__ __forceinline__ void issue(const MmaArgs &a, bool hold = false)
+    __device__ __forceinline__ void issue(const MmaArgs &a)
     {
         if (!have) return;
         const int off = (int)(ent >> 8 & 255ULL), len = (int)(ent & 255ULL);
         const int n = __shfl_sync(0xffffffffu, off + len, nseg - 1);
-        if (lane == 0 && !hold) {
+        if (lane == 0) {
             cnt[islot] = n;
             mbar_arrive_expect_tx(&full[islot], (uint32_t)(n * a.rowb));
         }
-        if (lane < nseg && !hold)
+        if (lane < nseg)
             bulk_g2s(ring + (islot * MM_SP + off) * a.rowb, a.rows + (size_t)(ent >> 16) * a.rowb,
                      (uint32_t)(len * a.rowb), &full[islot]);
         inflight++;
@@ -849,6 +847,41 @@ static int mma_chunks(int nsm, int nvdf, int warps, long long stages)
     return best;
 }
 
+// DGV_OPT_TEST_WITHHOLD: for one launch a segment of two pairs or more begins
+// one pair later, so that its stage's barrier, which expects the bytes up to
+// the last segment's end, waits for a pair that is not copied.  In the list and
+// not in the kernel: one more operand of the barriers' set-up there cost 0.5 %
+// at 27^3 (80.0 -> 80.4 ms for 4 VDFs).
+struct MmaWithhold {
+    unsigned long long *at = nullptr, was = 0;
+    int take(Ctx *c, const MmaList &M)
+    {
+        c->test_withhold = false;
+        int head[2] = {0, 0};
+        DGV_CUDA(c, cudaMemcpyAsync(head, M.sfirst, sizeof(head), cudaMemcpyDeviceToHost, c->stream));
+        DGV_CUDA(c, cudaStreamSynchronize(c->stream));
+        std::vector<unsigned long long> seg(head[1] - head[0]);  // the first stage's
+        unsigned long long *d = static_cast<unsigned long long *>(M.segs) + head[0];
+        DGV_CUDA(c, cudaMemcpyAsync(seg.data(), d, seg.size() * sizeof(was), cudaMemcpyDeviceToHost, c->stream));
+        DGV_CUDA(c, cudaStreamSynchronize(c->stream));
+        for (size_t k = 0; k < seg.size() && !at; k++)
+            if ((seg[k] & 255ULL) >= 2) {
+                was = seg[k];
+                at = d + k;
+                const unsigned long long later = was + (1ULL << 16) + (1ULL << 8) - 1ULL;
+                DGV_CUDA(c, cudaMemcpyAsync(at, &later, sizeof(later), cudaMemcpyHostToDevice, c->stream));
+                DGV_CUDA(c, cudaStreamSynchronize(c->stream));
+            }
+        return DGV_OK;
+    }
+    int give_back(Ctx *c)
+    {
+        DGV_CUDA(c, cudaMemcpyAsync(at, &was, sizeof(was), cudaMemcpyHostToDevice, c->stream));
+        DGV_CUDA(c, cudaStreamSynchronize(c->stream));
+        return DGV_OK;
+    }
+};
+
 typedef void (*MmaFn)(const MmaArgs);
 
 template <int P>
@@ -929,8 +962,8 @@ int collide_mma_device(Ctx *c, const double *d_f, const double *d_g, double *d_q
     a.units = (const MmaUnit *)pl->units; a.bounds = bounds;
     a.err = c->d_err; a.N = g.N; a.Nc = g.Nc; a.Mv = g.d.Mv; a.Mw = g.d.Mw; a.nchunks = nchunks;
     a.cell0 = cell0; a.ncell = cell1 - cell0; a.wait_ns = wait_limit_ns(c);
-    a.withhold = c->test_withhold ? 1 : 0;
-    c->test_withhold = false;
+    MmaWithhold wh;
+    if (c->test_withhold && (rc = wh.take(c, M))) return rc;
     MmaFn fn = g.P == 27 ? mma_pick<27>(f32, bil, gf) : mma_pick<8>(f32, bil, gf);
     DGV_CUDA(c, cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     KTimer kt(c);
@@ -942,6 +975,7 @@ int collide_mma_device(Ctx *c, const double *d_f, const double *d_g, double *d_q
         DGV_CUDA(c, cudaMemsetAsync(c->d_partial, 0, (size_t)nvdf * nchunks * len * sizeof(double), c->stream));
     }
     kt.stop(1);
+    if (wh.at && (rc = wh.give_back(c))) return rc;
     const long long nred = (long long)nvdf * ((long long)(len + 31) / 32);
     k_reduce_partials<<<(unsigned)nred, 256, 0, c->stream>>>(c->d_partial, c->d_nwt + (size_t)cell0 * g.P, d_q, nchunks,
                                                              (long long)len, nvdf, scale);

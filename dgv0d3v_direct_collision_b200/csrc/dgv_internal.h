@@ -195,7 +195,7 @@ struct Ctx {
     std::map<int, int> tc_tuned_adj;   // per batch class: the adjoint's persistent-launch choice
     double *d_tc2done = nullptr;       // persistent block-form launches: order flags (ints)
     size_t tc2done_bytes = 0;
-    bool test_withhold = false;   // DGV_OPT_TEST_WITHHOLD: the next launch of the block form, collide_mma.cu or adjoint_mma.cu withholds one copy
+    bool test_withhold = false;   // DGV_OPT_TEST_WITHHOLD: a wait of the next launch of the block form, collide_mma.cu or adjoint_mma.cu runs out
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> kt_pending, kt_pool;
     long long kt_launches = 0, kt_all = 0;
     double kt_ms = 0.0;

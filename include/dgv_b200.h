@@ -93,9 +93,9 @@ extern "C" {
                                  /* call on a grid of 8 or 27 nodes per cell  */
                                  /* (tensor cores in the block form, FP64,    */
                                  /* FP32-compensated, mixed terms, adjoint)   */
-                                 /* leaves one of its copies unissued, so its */
-                                 /* waits run out and it returns              */
-                                 /* DGV_ETIMEOUT; resets itself               */
+                                 /* waits for a copy or an arrival that does  */
+                                 /* not come, so its waits run out and it     */
+                                 /* returns DGV_ETIMEOUT; resets itself       */
 
 /* layouts for dgv_release_layouts */
 #define DGV_LAYOUT_F32 1      /* FP32 rows of the pair layout (FP32-compensated Q) and */

@@ -1,7 +1,7 @@
 """The bounded waits of the FP64 and FP32-compensated kernels, of the FP64
-adjoint and of the block form with eight nodes per cell: with one copy left
-unissued (DGV_OPT_TEST_WITHHOLD) the wait for it runs out, the call returns
-DGV_ETIMEOUT, and the same context then gives its earlier results."""
+adjoint and of the block form with eight nodes per cell: with a copy or an
+arrival withheld (DGV_OPT_TEST_WITHHOLD) the wait for it runs out, the call
+returns DGV_ETIMEOUT, and the same context then gives its earlier results."""
 import time
 
 import numpy as np
