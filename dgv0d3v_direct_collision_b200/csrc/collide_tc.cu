@@ -1251,10 +1251,19 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_collide_tc2(const __grid_cons
                 const T2Unit un = t2_unit<MG>(L, u);
                 const Tc2Args &a = L.g[MG ? un.gi : 0];
                 const int D0 = un.tile * NDG;
-                TcItem en = un.i0 < un.i1 ? a.items[un.i0] : TcItem{};
+                // eight nodes: an item is read one ahead of its use (14^3 x 150:
+                // 20.2 -> 18.9 ms; at 27 nodes that costs 2 % of a batch of one
+                // VDF tile, 21^3 x 37: 28.7 -> 29.3 ms, the mixed batch 47.7 -> 48.5)
+                TcItem en{};
+                if (P == 8 && un.i0 < un.i1) en = a.items[un.i0];
                 for (int it = un.i0; it < un.i1; it++) {
-                    const TcItem e = en;
-                    if (it + 1 < un.i1) en = a.items[it + 1];
+                    TcItem e;
+                    if constexpr (P == 8) {
+                        e = en;
+                        if (it + 1 < un.i1) en = a.items[it + 1];
+                    } else {
+                        e = a.items[it];
+                    }
                     const int s = q % NSLOT;
                     if (!mbar_wait<HOLD>(&s_empty[s], ((q / NSLOT) & 1) ^ 1, a.err, L.wait_ns)) { ok = false; break; }
                     // f of cells c1 + D - ccell (FP32) and c2 + D - ccell (fp16
