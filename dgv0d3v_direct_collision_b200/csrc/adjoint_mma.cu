@@ -21,7 +21,7 @@
 // bulk copies of its own.
 //
 // Measured (B200, 1965 MHz), one VDF at 21^3: 44.9 ms with one cell per lane,
-// 5.6 ms here.  The products take 2.4 ms of that (76 % of a tile's pairs are
+// 5.5 ms here (27^3: 260 -> 40.5).  The products take 2.4 ms of that (76 % of a tile's pairs are
 // real: a block has ~16 pairs per l1); shared memory delivers 63 % of its words
 // and the warps' own dependent steps per tile fill the rest, so four warps per
 // scheduler with two row tiles are faster than two with three (6.8 ms, also

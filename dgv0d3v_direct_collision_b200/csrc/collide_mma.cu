@@ -25,21 +25,23 @@
 // robin to the warps, each warp streaming its own through a ring; at the end
 // of a unit the warps' sums are added in a fixed order and once into the CTA's
 // partial Q.  Ranges hold equal work and may be cut anywhere, so one wave of
-// CTAs is balanced (the longest within 2.6 % of the mean at 27^3);
+// CTAs is balanced (the longest within 2.6 % of the mean at 27^3, 5 to 6 % at
+// 15^3 and 21^3 and at 20^3 with eight nodes, whose costs are those of 27);
 // k_reduce_partials adds the ranges in a fixed order: results are the same
 // from run to run.
 //
 // What bounds it (B200, 1965 MHz): the FP64 tensor pipe, 80 % busy at 27^3,
-// 77 % at 21^3, 69 % at 15^3 (148 ranges of three boxes each, and 680 cycles a
+// 76 % at 21^3, 67 % at 15^3 (148 ranges of three boxes each, and 680 cycles a
 // tile at a unit's end).  A stage of 8 tiles takes 605 SM cycles, 512 of them
 // products; the rest is the gathers' latency, which two warps per scheduler
 // hide but for those 93.  Tried: explicit double buffering of the gathers
 // across steps and stages (620-730, more registers and spills), 12 warps of 6
 // or 5 tiles and 16 of 4 (the same share), 32 pairs a stage (2 % faster, no
 // room at 27^3).  Per VDF, one lane per cell -> this kernel: 27^3 129.7 -> 20.1
-// ms, 21^3 mixed terms 32.1 -> 3.2 ms, 15^3 with projection 1.98 -> 0.28 ms.
+// ms, 21^3 mixed terms 32.1 -> 3.2 ms, 15^3 with projection 1.95 -> 0.285 ms.
 // Eight nodes per cell leave one column tile per product: shared-memory
-// gathers bound it (27 % of the tensor pipe).
+// gathers bound it (20^3: 31 % of the tensor pipe, 60 % of shared memory's
+// words; 13.5 -> 2.7 ms per VDF).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -447,7 +449,9 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_collide_mma(const __grid_cons
 // and the shuffles' ~21 words per pair and their latency bound it (scalar: two
 // rows and all columns per lane 655, but rows in steps of 32; 12 or 16 warps of
 // 32 rows 405 per 32 rows).  Per Q at 21^3 with projection, one cell per lane ->
-// this kernel: 18.3 -> 3.3 ms.
+// this kernel: 18.3 -> 3.3 ms.  The FP64 kernel above has become the faster one
+// all the same (one VDF, FP64 / FP32: 15^3 0.27 / 0.38 ms, 21^3 2.98 / 3.34,
+// 27^3 20.4 / 23.0; eight nodes 14^3 0.24 / 0.29, 20^3 2.7 / 3.6).
 constexpr int FC_WARPS = 8, FC_THREADS = 32 * FC_WARPS;
 constexpr int FC_TILE = 16, FC_MT = 4;  // rows per tile (A = 2 per tile); tiles per unit
 
@@ -909,6 +913,8 @@ int collide_mma_device(Ctx *c, const double *d_f, const double *d_g, double *d_q
     int rc;
     if (f32 && (rc = ensure_rows32(c))) return rc;  // rebuilt if released
     // costs fitted to the measured cycles of the ranges at 15^3, 21^3 and 27^3
+    // (27 nodes); at eight nodes, 20^3, they leave the longest range 5 % above
+    // the mean, as at 21^3
     const MmaShape S = f32 ? MmaShape{FC_TILE, FC_MT, 125, 235, 3000, 1500} : MmaShape{8, MM_MT, 66, 80, 3000, 600};
     MmaList &M = f32 ? L.groups : L.mma;
     MmaPlan *pl = nullptr;

@@ -816,8 +816,9 @@ static int tc_lists(Ctx *c, int NDG, TcLists *out)
 // role, less than the latency of its copies, so what shared and tensor memory
 // the small tiles leave goes to four item slots, eight W stages and eight
 // accumulators of 64 columns, and the producer loads an item one ahead.  With
-// long holds in the waits (HOLD below) 14^3 x 150 takes 19.0 ms, 20.9 in the
-// tiles of 27 nodes: an item's chain of waits bounds it, ~2,000 cycles.
+// long holds in the waits (HOLD below) 14^3 x 150 takes 18.95 ms; in the tiles
+// of 27 nodes 20.3 without holds, 20.5 with: an item's chain of waits bounds it,
+// ~2,000 cycles.
 __host__ __device__ constexpr int t2_n(int P) { return P == 8 ? 64 : 256; }        // columns (l1, p) per group
 __host__ __device__ constexpr int t2_k(int P) { return P == 8 ? 16 : 32; }         // nodes l2 per block, zero-padded
 __host__ __device__ constexpr int t2_tile(int P) { return t2_n(P) * t2_k(P) * 2; }  // one fp16 tile (16 KiB; 2 KiB)
@@ -1156,9 +1157,11 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_collide_tc2(const __grid_cons
     constexpr int NDG = TC_ROWS / VB;
     constexpr int NG = t2_groups(P), T2_N = t2_n(P), T2_K = t2_k(P), T2_TILE = t2_tile(P), T2_GREC = t2_grec(P);
     constexpr int T2_ATILE = t2_atile(P), T2_NSTW = t2_nstw(P), NSLOT = t2_nslot(P), NACC = t2_nacc(P);
-    // Long holds suit the short items of 8 nodes per cell (14^3 x 150: 20.8 ms
-    // with the default, 19.0 with 50 us) and not those of 27 (27^3 x 256: 537 ms
-    // with the default, 546 with 50 us)
+    // Long holds suit the short items of 8 nodes per cell in their own tiles
+    // (14^3 x 150: 20.8 ms with the default, 18.95 with 50 us; in the tiles of
+    // 27 nodes 20.3 and 20.5) and not those of 27 (27^3 x 256: 537 ms with the
+    // default, 546 with 50 us).  A wait limit (DGV_OPT_WAIT_LIMIT_US) below a
+    // hold is kept to within one.
     constexpr uint32_t HOLD = P == 8 ? 50000 : 0;
     constexpr int SBO = 16 * T2_K;  // row groups of 8 of a tile
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -1339,7 +1342,8 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_collide_tc2(const __grid_cons
         // value; with the warp converged they are uniform, and the issuer keeps
         // up with the tensor pipe beside the epilogue warps of its scheduler
         // (B200, 21^3 x 37: 32.1 -> 29.2 ms, 14^3 x 150, 8 nodes: 22.4 -> 20.9,
-        // 27^3 x 256: 543 -> 538, adjoint 21^3 x 150: 150.8 -> 147.9).
+        // adjoint 21^3 x 150: 150.8 -> 147.9; 27^3 x 256 the same to within its
+        // runs, 536-543).
         {
             // FP32 accumulator, fp16 A and B, both K-major, M = 128, N = 256;
             // an item's last group holds ncol - 256 (ngb-1) columns: its MMAs

@@ -302,8 +302,8 @@ class DGVSolver:
 
     def vjp(self, f, v, out=None, precision="f64"):
         """g = J(f)^T v for one VDF or a batch [nb, N] (dgv_vjp_batched);
-        precision "f64" (FP64 kernel per VDF) or "tc" (block form on the
-        tensor cores, all VDFs in one pass)."""
+        precision "f64" or "tc" (block form on the tensor cores); all VDFs
+        in one pass."""
         _check_f64(f); _check_f64(v)
         if tuple(f.shape) != tuple(v.shape) or f.shape[-1] != self.N:
             raise ValueError("vjp: f and v must have the same shape [..., N]")

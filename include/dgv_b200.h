@@ -51,7 +51,9 @@ extern "C" {
 
 /* options for dgv_set_option */
 #define DGV_OPT_PROJECT 1  /* 1: apply the FP64 conservation projection to Q  */
-#define DGV_OPT_NCHUNKS 2  /* work chunks per VDF (0 = autotune)             */
+#define DGV_OPT_NCHUNKS 2  /* work chunks per VDF (0 = the library's choice: */
+                           /* by a rule on the batch and the SMs, with 1 or   */
+                           /* 125 nodes per cell measured for small batches)  */
 #define DGV_OPT_KTIMING 3  /* 1: time the collision kernel with CUDA events   */
                            /* on the context stream (read: dgv_kernel_stats)  */
 #define DGV_OPT_TCFORM 4   /* tensor-core form: 2 (default) = dense cell-pair */
@@ -70,7 +72,8 @@ extern "C" {
                                  /* of a collision kernel (block form, FP64,  */
                                  /* FP32-compensated, mixed terms, adjoint)   */
                                  /* gives up (0 = 4 s); the call then returns */
-                                 /* DGV_ETIMEOUT                              */
+                                 /* DGV_ETIMEOUT.  The tensor-core path of 8  */
+                                 /* nodes per cell looks every 50 us          */
 #define DGV_OPT_TCAUTOTUNE 9      /* block form: 1 (default) = on the first    */
                                  /* evaluation of each batch class, time VDF  */
                                  /* tiles per CTA x records per launch x      */
@@ -83,8 +86,10 @@ extern "C" {
                                  /* each set's sums added in set order; 0 =   */
                                  /* one launch per set (same results, bit for */
                                  /* bit)                                      */
-#define DGV_OPT_FGLOBAL 10        /* CUDA-core kernels (FP64, FP32-compensated, */
-                                 /* mixed terms, FP64 adjoint): 0 (default) = */
+#define DGV_OPT_FGLOBAL 10        /* FP64 and FP32-compensated Q, mixed terms   */
+                                 /* (and the FP64 adjoint with 1 or 125 nodes */
+                                 /* per cell; with 8 or 27 it always reads    */
+                                 /* the caller's f): 0 (default) =            */
                                  /* f of a VDF staged in shared memory when   */
                                  /* it fits, else gathered from a local-major */
                                  /* copy in global memory (L1/L2); 1 = always */
@@ -142,7 +147,8 @@ int dgv_get_option(dgv_ctx *ctx, int option, int64_t *value);
  * the change in the device's free memory.  No counterpart in the reference. */
 int dgv_release_layouts(dgv_ctx *ctx, int mask, int64_t *freed_bytes);
 /* No counterpart in the reference (measurement hook): summed device time in
- * ms and launch count of the collision kernel (k_collide_tc / k_collide_pipe)
+ * ms and launch count of the collision kernel (k_collide_tc2, k_collide_tc,
+ * k_collide_mma, k_collide_f32 or k_collide_pipe)
  * over the calls made since the last reset while DGV_OPT_KTIMING was on,
  * and the number of kernels of this library those calls launched.
  * Synchronises on the recorded events; reset != 0 clears the sums. */
@@ -281,7 +287,9 @@ int dgv_collide_cells(dgv_ctx *ctx, int32_t nb, const double *f, double *q, int3
  * DGV_EINVAL.  All calls share the array and leave their partial sums in it:
  * calls that overlap on the GPU (other streams or host threads) race, so
  * serialise them.  No conservation projection.  stream NULL = the context's
- * stream. */
+ * stream.  It keeps one output cell per lane and no work lists, which would
+ * have to be allocated: on grids of 8 or 27 nodes per cell it takes 7 to 34
+ * times as long as dgv_collide in FP64 (one VDF, 27^3: 470 ms against 20). */
 int dgv_collide_f64_noalloc(dgv_ctx *ctx, const double *f, double *q, int32_t nb, void *stream);
 
 /* -- time integration ------------------------------------------------------ */
